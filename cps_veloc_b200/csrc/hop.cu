@@ -3,80 +3,16 @@
 #include <cstring>
 
 #include "cpsgpu_impl.h"
-#include "hop.cuh"
+#include "hop_pick.cuh"
 #include "tune.h"
 
 namespace cpsgpu {
 
 namespace {
 
-using HopFn = void (*)(const HopParams, const HopViews, SolverScalars *, double *);
-
-bool g_dag = false;  // set by launch_hop before pick()
-int g_ns = 1;        // slices per thread (2: DWF slice pairs)
-
-template <int P, int RECON, int EP, int PR, int PX>
-HopFn get() {
-  // FP32 arithmetic only: the FP64 pair kernel spills kilobytes
-  if constexpr (!ep_mix(EP) && P != PREC_DOUBLE) {
-    if (g_ns == 2)
-      return g_dag ? hop_kernel<P, RECON, EP, PR, PX, true, false, 2> : hop_kernel<P, RECON, EP, PR, PX, false, false, 2>;
-  }
-  return g_dag ? hop_kernel<P, RECON, EP, PR, PX, true> : hop_kernel<P, RECON, EP, PR, PX, false>;
-}
-
-template <int P, int RECON>
-HopFn pick_ep(int ep, int pr, int px) {
-  constexpr int PXS = (P == PREC_DOUBLE) ? PREC_DOUBLE : PREC_SINGLE;
-  switch (ep) {
-    case EP_STORE: return get<P, RECON, EP_STORE, P, P>();
-    case EP_AXPY: return get<P, RECON, EP_AXPY, P, P>();
-    case EP_MIX: return get<P, RECON, EP_MIX, P, P>();
-    case EP_MIX_AXPY: return get<P, RECON, EP_MIX_AXPY, P, P>();
-    case EP_CG:
-      if (pr == P && px == PXS) return get<P, RECON, EP_CG, P, PXS>();
-      break;
-    case EP_MIX_CG:
-      if (pr == P && px == PXS) return get<P, RECON, EP_MIX_CG, P, PXS>();
-      break;
-    case EP_RES:
-    case EP_MIX_RES:
-      if constexpr (P == PREC_DOUBLE) {
-        if (ep == EP_RES) {
-          if (pr == PREC_DOUBLE) return get<P, RECON, EP_RES, PREC_DOUBLE, P>();
-          if (pr == PREC_SINGLE) return get<P, RECON, EP_RES, PREC_SINGLE, P>();
-          if (pr == PREC_HALF) return get<P, RECON, EP_RES, PREC_HALF, P>();
-        } else {
-          if (pr == PREC_DOUBLE) return get<P, RECON, EP_MIX_RES, PREC_DOUBLE, P>();
-          if (pr == PREC_SINGLE) return get<P, RECON, EP_MIX_RES, PREC_SINGLE, P>();
-          if (pr == PREC_HALF) return get<P, RECON, EP_MIX_RES, PREC_HALF, P>();
-        }
-      }
-      break;
-  }
-  throw Error(-2, "hop: unsupported epilogue/precision combination");
-}
-
-HopFn pick(int prec, int recon, int ep, int pr, int px) {
-  if (prec == PREC_DOUBLE) return recon == 18 ? pick_ep<PREC_DOUBLE, 18>(ep, pr, px) : pick_ep<PREC_DOUBLE, 12>(ep, pr, px);
-  if (prec == PREC_SINGLE) return recon == 18 ? pick_ep<PREC_SINGLE, 18>(ep, pr, px) : pick_ep<PREC_SINGLE, 12>(ep, pr, px);
-  if (recon == LINK_F32_18) return pick_ep<PREC_HALF, LINK_F32_18>(ep, pr, px);
-  if (recon == LINK_F32_12) return pick_ep<PREC_HALF, LINK_F32_12>(ep, pr, px);
-  return recon == 18 ? pick_ep<PREC_HALF, 18>(ep, pr, px) : pick_ep<PREC_HALF, 12>(ep, pr, px);
-}
-
-// the t-slab decomposition's hops (store epilogue, FP64 / FP32)
-HopFn pick_halo(int prec, int recon) {
-  if (recon != 12 && recon != 18) throw Error(-2, "decomposed hop: 12- or 18-real links");
-  if (prec == PREC_DOUBLE)
-    return recon == 12 ? (g_dag ? hop_kernel<PREC_DOUBLE, 12, EP_STORE, PREC_DOUBLE, PREC_DOUBLE, true, true>
-                                : hop_kernel<PREC_DOUBLE, 12, EP_STORE, PREC_DOUBLE, PREC_DOUBLE, false, true>)
-                       : (g_dag ? hop_kernel<PREC_DOUBLE, 18, EP_STORE, PREC_DOUBLE, PREC_DOUBLE, true, true>
-                                : hop_kernel<PREC_DOUBLE, 18, EP_STORE, PREC_DOUBLE, PREC_DOUBLE, false, true>);
-  return recon == 12 ? (g_dag ? hop_kernel<PREC_SINGLE, 12, EP_STORE, PREC_SINGLE, PREC_SINGLE, true, true>
-                              : hop_kernel<PREC_SINGLE, 12, EP_STORE, PREC_SINGLE, PREC_SINGLE, false, true>)
-                     : (g_dag ? hop_kernel<PREC_SINGLE, 18, EP_STORE, PREC_SINGLE, PREC_SINGLE, true, true>
-                              : hop_kernel<PREC_SINGLE, 18, EP_STORE, PREC_SINGLE, PREC_SINGLE, false, true>);
+HopFn pick(int prec, const HopSel &q) {
+  if (q.halo && q.recon != 12 && q.recon != 18) throw Error(-2, "decomposed hop: 12- or 18-real links");
+  return prec == PREC_DOUBLE ? pick_hop_double(q) : prec == PREC_SINGLE ? pick_hop_single(q) : pick_hop_half(q);
 }
 
 size_t real_size(int prec) { return prec == PREC_DOUBLE ? 8 : 4; }
@@ -140,10 +76,9 @@ void launch_hop(const Dirac &D, const HopLaunch &L, const SpinorView &in, const 
   TuneKey key{L.prec, recon, L.ep, D.kind, D.ls};
   dim3 block = hop_block(key, mix);
   // block.z of a tuned shape: slices per thread (2: DWF slice pairs)
-  g_ns = (block.z == 2 && hp.dwf && !mix && !halo && L.prec != PREC_DOUBLE && D.ls % (4 * (int)block.y) == 0) ? 2 : 1;
+  const int ns = (block.z == 2 && hp.dwf && !mix && !halo && L.prec != PREC_DOUBLE && D.ls % (4 * (int)block.y) == 0) ? 2 : 1;
   block.z = 1;
-  g_dag = (L.dag != 0);
-  HopFn fn = halo ? pick_halo(L.prec, recon) : pick(L.prec, recon, L.ep, L.pr, L.px);
+  HopFn fn = pick(L.prec, HopSel{recon, L.ep, L.pr, L.px, L.dag != 0, ns, halo});
   unsigned nsb;
   if (L.sub == SUB_BOUNDARY) {
     hp.subn = (hp.face + (int)block.x - 1) / (int)block.x;
@@ -158,7 +93,7 @@ void launch_hop(const Dirac &D, const HopLaunch &L, const SpinorView &in, const 
     hp.i0 = (L.sub == SUB_INTERIOR) ? hp.face : 0;
     hp.iend = hp.i0 + (int)nsites;
   }
-  hp.nsg = g_ns == 2 ? D.ls / (2 * (int)block.y) : (D.ls + block.y - 1) / block.y;
+  hp.nsg = ns == 2 ? D.ls / (2 * (int)block.y) : (D.ls + block.y - 1) / block.y;
   // ORDER_SITES: the slice groups on the grid's y (blocks run x fastest)
   const bool sites_first = (hop_order(key) == ORDER_SITES && hp.nsg > 1);
   hp.spar = (hp.dwf && !mix && block.y > 1 && D.ls % (2 * block.y) == 0) ? 1 : 0;
