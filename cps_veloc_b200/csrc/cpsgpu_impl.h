@@ -150,6 +150,7 @@ struct CachedGraph {
 struct MsWork {
   Field chi, r, tmp;
   std::vector<Field> p, psi;
+  std::vector<Field> ring;  // residuals of a chunk's iterations (deferred updates); the last is r
   DeviceBuffer st, ms, pv, psiv;
   OpWork w;
   // the recurrences' loop: a WHILE node over chunks of iterations, ctl its

@@ -110,7 +110,7 @@ struct HopParams {
 
 struct HopViews {
   GaugeView U;
-  SpinorView in, out, x;  // hop input, output, axpby source
+  SpinorView in, out, x;  // hop input, output (CG: where the new residual goes, null = r), axpby source
   SpinorView r, sol, p;   // CG / RES epilogue fields
   SpinorView b;           // RES: right-hand side (double)
   // t halos, [slice][12 reals][face] in the hop's precision: hf from the
@@ -349,6 +349,11 @@ __device__ __forceinline__ void hop_epilogue(const HopParams &hp, const HopViews
       RR rfull[PR == PREC_HALF ? 24 : 1];
       ChunkReader<P> xr(v.x, sl, i);
       ChunkReader<PR> pr(v.p, sl, i), rr(v.r, sl, i);
+      SpinorView rnew = v.r;
+      if (v.out.data) {
+        rnew.data = v.out.data;
+        rnew.norm = v.out.norm;
+      }
 #pragma unroll
       for (int c = 0; c < 6; c++) {
         R xv[4];
@@ -366,7 +371,7 @@ __device__ __forceinline__ void hop_epilogue(const HopParams &hp, const HopViews
 #pragma unroll
           for (int k = 0; k < 4; k++) rfull[4 * c + k] = rv[k];
         } else {
-          Chunk4<PR>::store(v.r, sl, i, c, rv);
+          Chunk4<PR>::store(rnew, sl, i, c, rv);
         }
         if (with_sol) {
           RX sv[4];
@@ -376,7 +381,7 @@ __device__ __forceinline__ void hop_epilogue(const HopParams &hp, const HopViews
           if constexpr (PX != PREC_HALF) Chunk4<PX>::store(v.sol, sl, i, c, sv);
         }
       }
-      if constexpr (PR == PREC_HALF) SpinorIO<PR>::store(v.r, sl, i, rfull);
+      if constexpr (PR == PREC_HALF) SpinorIO<PR>::store(rnew, sl, i, rfull);
     }
     red[0] += double(n_r);
   } else if constexpr (ep_res(EP)) {

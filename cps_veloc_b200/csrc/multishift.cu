@@ -3,10 +3,11 @@
 // One iteration is: the M half of MatPcDagMatPc on p_0 (reducing <p,(A+m_0)p>,
 // whose last block runs the shifted z / beta recurrences for every shift),
 // the M^dagger half with the residual update r += b A p_0 and |r|^2 fused in
-// (last block: per-shift convergence), then one kernel that updates psi_s
-// and p_s of every shift still running (a thread per site and shift; a thread
-// per site summing over the shifts when only the weighted sum is kept).  The
-// scalars never leave the device.
+// (last block: per-shift convergence), then the updates of psi_s and p_s of
+// every shift still running.  Only p_0 feeds the next operator application,
+// so shift 0 is updated in every iteration and the others once per
+// MS_DEFER iterations (ms_flush_kernel), from the residuals and coefficients
+// of those iterations.  The scalars never leave the device.
 //
 // precision CPSGPU_SINGLE runs the recurrences on FP32 vectors, the
 // solutions included (the per-shift update then moves half the bytes of the
@@ -122,12 +123,172 @@ __global__ void __launch_bounds__(128) ms_update_shift_kernel(SpinorView r, cons
   }
 }
 
-__global__ void ms_mark_kernel(MsScalars *ms) { ms->upd_done_iter = ms->k; }
+// ---- deferred updates
+// The recurrences of the shifts s > 0 are elementwise over the field and read
+// only r besides their own vectors, so MS_DEFER iterations can be applied at
+// once: r^0 .. r^7 of the chunk are kept (a ring of residual fields) and one
+// pass over p_s and psi_s does for every element what the iterations did,
+// in the same order.  Per iteration the pass moves (4 (n-1) + 8) / 8 vectors
+// where the per-iteration update moved 4 (n-1) + 1; it is HBM bound.
+// Measured: see the launch rule in minvcg().
+
+template <int P> struct MsVec;  // one 16-byte element of a field
+template <> struct MsVec<PREC_DOUBLE> {
+  using T = double2;
+  static constexpr int N = 2;
+  static __device__ __forceinline__ void get(T q, double *v) { v[0] = q.x; v[1] = q.y; }
+  static __device__ __forceinline__ T put(const double *v) { return make_double2(v[0], v[1]); }
+};
+template <> struct MsVec<PREC_SINGLE> {
+  using T = float4;
+  static constexpr int N = 4;
+  static __device__ __forceinline__ void get(T q, float *v) { v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w; }
+  static __device__ __forceinline__ T put(const float *v) { return make_float4(v[0], v[1], v[2], v[3]); }
+};
+
+struct MsRing {
+  const void *r[MS_DEFER];  // the residual of each iteration of a chunk
+};
+
+// shift 0 of the chunk's iteration `slot` (p_0 is the next operator's input):
+// psi_0 += f p_0, p_0 = r + a p_0; nothing when that iteration did not run
+template <int P>
+__global__ void __launch_bounds__(256) ms_lead_kernel(const void *r, void *p0, void *psi0, const MsScalars *ms, int slot,
+                                                       size_t n) {
+  using V = MsVec<P>;
+  if (ms->nh != slot + 1) return;
+  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= n) return;
+  const bool upd = ms->h_upd[slot][0], adv = ms->h_adv[slot][0];
+  typename V::T *pp = reinterpret_cast<typename V::T *>(p0) + idx, *yp = reinterpret_cast<typename V::T *>(psi0) + idx;
+  RealT<P> p[V::N], y[V::N], rv[V::N];
+  V::get(*pp, p);
+  if (upd) V::get(*yp, y);
+  if (adv) V::get(__ldg(reinterpret_cast<const typename V::T *>(r) + idx), rv);
+  if (upd) {
+    const double f = ms->hf[slot][0];
+#pragma unroll
+    for (int k = 0; k < V::N; k++) y[k] = RealT<P>(double(y[k]) + f * double(p[k]));
+    *yp = V::put(y);
+  }
+  if (adv) {
+    const RealT<P> a = RealT<P>(ms->ha[slot][0]);
+#pragma unroll
+    for (int k = 0; k < V::N; k++) p[k] = rv[k] + a * p[k];
+    *pp = V::put(p);
+  }
+}
+
+// the shifts s > 0 over the iterations since the last flush.  A thread per
+// 16-byte element: its MS_DEFER residuals stay in registers while it walks
+// the shifts, the next shift's vectors loaded before the current one's
+// arithmetic.  SUM: one solution, psi_0 += sum_s f_s p_s (type SINGLE).
+template <int P, bool SUM>
+__global__ void __launch_bounds__(256) ms_flush_kernel(const MsRing ring, const SpinorView *pv, const SpinorView *psiv,
+                                                       const MsScalars *ms, size_t n) {
+  using V = MsVec<P>;
+  using T = typename V::T;
+  using R = RealT<P>;
+  const int nh = ms->nh, ns = ms->nshift;
+  if (nh == 0) return;
+  __shared__ double f[MS_DEFER][MS_MAX];
+  __shared__ R z[MS_DEFER][MS_MAX], a[MS_DEFER][MS_MAX];
+  __shared__ unsigned upd[MS_MAX], adv[MS_MAX];
+  __shared__ T *pp[MS_MAX], *yp[MS_MAX];
+  for (int s = threadIdx.x; s < ns; s += blockDim.x) {
+    unsigned u = 0, d = 0;
+    for (int j = 0; j < nh; j++) {
+      u |= (unsigned)ms->h_upd[j][s] << j;
+      d |= (unsigned)ms->h_adv[j][s] << j;
+    }
+    upd[s] = u;
+    adv[s] = d;
+    pp[s] = reinterpret_cast<T *>(pv[s].data);
+    yp[s] = SUM ? nullptr : reinterpret_cast<T *>(psiv[s].data);
+  }
+  for (int q = threadIdx.x; q < nh * ns; q += blockDim.x) {
+    const int j = q / ns, s = q % ns;
+    f[j][s] = ms->hf[j][s];
+    z[j][s] = R(ms->hz[j][s]);
+    a[j][s] = R(ms->ha[j][s]);
+  }
+  __syncthreads();
+  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= n) return;
+  R r[MS_DEFER][V::N];
+#pragma unroll
+  for (int j = 0; j < MS_DEFER; j++)
+    if (j < nh) V::get(__ldg(reinterpret_cast<const T *>(ring.r[j]) + idx), r[j]);
+  double sum[V::N];
+  T *const s0 = reinterpret_cast<T *>(psiv[0].data) + idx;
+  if constexpr (SUM) {
+    R y[V::N];
+    V::get(*s0, y);
+#pragma unroll
+    for (int k = 0; k < V::N; k++) sum[k] = double(y[k]);
+  }
+  auto next = [&](int s) {
+    while (s < ns && !(upd[s] | adv[s])) s++;
+    return s;
+  };
+  int s = next(1);
+  T pq, yq;
+  if (s < ns) {
+    pq = pp[s][idx];
+    if (!SUM) yq = yp[s][idx];
+  }
+  while (s < ns) {
+    const int t = next(s + 1);
+    T pn, yn;
+    if (t < ns) {
+      pn = pp[t][idx];
+      if (!SUM) yn = yp[t][idx];
+    }
+    R p[V::N], y[V::N];
+    V::get(pq, p);
+    if (!SUM) V::get(yq, y);
+    const unsigned u = upd[s], d = adv[s];
+#pragma unroll
+    for (int j = 0; j < MS_DEFER; j++) {
+      if ((u >> j) & 1) {
+        const double fj = f[j][s];
+#pragma unroll
+        for (int k = 0; k < V::N; k++) {
+          if constexpr (SUM) sum[k] += fj * double(p[k]);
+          else y[k] = R(double(y[k]) + fj * double(p[k]));
+        }
+      }
+      if ((d >> j) & 1) {
+        const R zj = z[j][s], aj = a[j][s];
+#pragma unroll
+        for (int k = 0; k < V::N; k++) p[k] = zj * r[j][k] + aj * p[k];
+      }
+    }
+    if (d) pp[s][idx] = V::put(p);
+    if (!SUM && u) yp[s][idx] = V::put(y);
+    pq = pn;
+    yq = yn;
+    s = t;
+  }
+  if constexpr (SUM) {
+    R y[V::N];
+#pragma unroll
+    for (int k = 0; k < V::N; k++) y[k] = R(sum[k]);
+    *s0 = V::put(y);
+  }
+}
+
+// the end of an iteration whose updates were applied at once
+__global__ void ms_mark_kernel(MsScalars *ms) {
+  ms->upd_done_iter = ms->k;
+  ms->nh = 0;
+}
 
 // the condition of the recurrences' WHILE node, after each chunk: another
 // chunk while the solve runs, never more than ctl[1] chunks (ctl[0] counts)
-__global__ void ms_loop_cond_kernel(cudaGraphConditionalHandle h, const SolverScalars *st, int *ctl) {
+__global__ void ms_loop_cond_kernel(cudaGraphConditionalHandle h, const SolverScalars *st, MsScalars *ms, int *ctl) {
   if (threadIdx.x != 0) return;
+  ms->nh = 0;  // the chunk's updates are flushed
   const int bodies = ++ctl[0];
   cudaGraphSetConditional(h, (st->done == 0 && bodies < ctl[1]) ? 1u : 0u);
 }
@@ -254,9 +415,39 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
   CPSGPU_CUDA(cudaMemcpyAsync(pvd.ptr, pv.data(), sizeof(SpinorView) * nshift, cudaMemcpyHostToDevice, s));
   CPSGPU_CUDA(cudaMemcpyAsync(psivd.ptr, psiv.data(), sizeof(SpinorView) * npsi, cudaMemcpyHostToDevice, s));
 
+  // The deferred updates' ring of residuals (mw.ring and r itself, the last
+  // slot).  From 3 shifts on: with 2 the flush reads as much as it saves.
+  // Seven more vectors beside the 2 n + 5 of the workspace, taken only while
+  // they are a small part of the free memory; else every iteration updates
+  // every shift.  Measured, the
+  // whole call: n = 16 summed, Wilson 24^3x48 FP64, 63.3 -> 52.9 ms (12.6 ms
+  // of it upload); n = 10, DWF 12^3x24 Ls=8 FP64, 74.4 -> 54.0 ms (23 ms of
+  // it host copies)
+  bool deferred = false;
+  auto ensure_ring = [&] {
+    if (nshift < 3) return;
+    const size_t one_field = r.data.bytes;
+    const bool have = mw.ring.size() == MS_DEFER - 1 && mw.ring[0].data.ptr && mw.ring[0].prec == P &&
+                      mw.ring[0].vh == vh && mw.ring[0].ls == ls;
+    if (!have) {
+      mw.ring.clear();
+      size_t free_b = 0, total_b = 0;
+      CPSGPU_CUDA(cudaMemGetInfo(&free_b, &total_b));
+      if ((MS_DEFER - 1) * one_field > free_b / 4) return;
+      mw.ring.resize(MS_DEFER - 1);
+      for (auto &f : mw.ring) f.create(P, vh, ls, 1);
+    }
+    deferred = true;
+  };
+  const size_t per = (size_t)vh * ls;
+  const size_t nvec = per * (P == PREC_DOUBLE ? 12 : 6);  // 16-byte elements of a field
+  auto slot_r = [&](int slot) { return slot == MS_DEFER - 1 ? r.view() : mw.ring[slot].view(); };
+
   // one iteration: M half (reduce <p,(A+m0)p>), M^dagger half with the
-  // residual update, then the per-shift vector updates.
-  auto iteration = [&](int use_chi) {
+  // residual update, then the vector updates: of every shift (slot < 0), or
+  // of shift 0 in iteration `slot` of a chunk whose other shifts are flushed
+  // at its end
+  auto iteration = [&](int use_chi, int slot) {
     const bool mob = (D.kind == KIND_MOBIUS);
     HopLaunch Lh;
     Lh.prec = P;
@@ -307,8 +498,17 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
     Lh.pr = P;
     Lh.px = px_of(P);
     Lh.ep = mix_last ? EP_MIX_CG : EP_CG;
+    if (slot >= 0) {
+      const SpinorView rnew = slot_r(slot);
+      launch_hop(D, Lh, hop_in, rnew, x, slot_r((slot + MS_DEFER - 1) % MS_DEFER), SpinorView(), in, SpinorView(), st);
+      const unsigned g = (unsigned)((nvec + 255) / 256);
+      if (P == PREC_DOUBLE) ms_lead_kernel<PREC_DOUBLE><<<g, 256, 0, s>>>(rnew.data, p[0].data.ptr, psi[0].data.ptr, msd, slot, nvec);
+      else ms_lead_kernel<PREC_SINGLE><<<g, 256, 0, s>>>(rnew.data, p[0].data.ptr, psi[0].data.ptr, msd, slot, nvec);
+      CPSGPU_CUDA(cudaGetLastError());
+      launch_counter()++;
+      return;
+    }
     launch_hop(D, Lh, hop_in, SpinorView(), x, r.view(), SpinorView(), in, SpinorView(), st);
-    size_t per = (size_t)vh * ls;
     if (dev_type != 0) {
       const unsigned g = (unsigned)((per + 127) / 128) * (unsigned)nshift;
       if (P == PREC_DOUBLE)
@@ -327,15 +527,33 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
     ms_mark_kernel<<<1, 1, 0, s>>>(msd);
     CPSGPU_CUDA(cudaGetLastError());
   };
+  // the other shifts' updates of a chunk's iterations
+  auto flush = [&] {
+    MsRing ring;
+    for (int j = 0; j < MS_DEFER; j++) ring.r[j] = slot_r(j).data;
+    const unsigned g = (unsigned)((nvec + 255) / 256);
+    if (dev_type == 0) {
+      ms_flush_kernel<PREC_DOUBLE, true><<<g, 256, 0, s>>>(ring, pvd.as<SpinorView>(), psivd.as<SpinorView>(), msd, nvec);
+    } else if (P == PREC_DOUBLE) {
+      ms_flush_kernel<PREC_DOUBLE, false><<<g, 256, 0, s>>>(ring, pvd.as<SpinorView>(), psivd.as<SpinorView>(), msd, nvec);
+    } else {
+      ms_flush_kernel<PREC_SINGLE, false><<<g, 256, 0, s>>>(ring, pvd.as<SpinorView>(), psivd.as<SpinorView>(), msd, nvec);
+    }
+    CPSGPU_CUDA(cudaGetLastError());
+    launch_counter()++;
+  };
 
   CPSGPU_CUDA(cudaStreamSynchronize(s));
   const clk::time_point t_rec = clk::now();
-  const int chunk = 8;
+  constexpr int chunk = MS_DEFER;
   mw.ctl.ensure(2 * sizeof(int));
   const int hctl[2] = {0, (int)std::min<long>((long)max_num_iter / chunk + 4, 1L << 30)};
-  const std::vector<long long> key = {P, nshift, dev_type, L.recon(P), D.pc_type, D.cplx ? 1 : 0,
-                                      (long long)(size_t)r.data.ptr, (long long)(size_t)w.t1.data.ptr,
-                                      (long long)(size_t)p[0].data.ptr, (long long)(size_t)psi[0].data.ptr};
+  auto graph_key = [&]() -> std::vector<long long> {
+    return {P, nshift, dev_type, L.recon(P), D.pc_type, D.cplx ? 1 : 0,
+            (long long)(size_t)r.data.ptr, (long long)(size_t)w.t1.data.ptr,
+            (long long)(size_t)p[0].data.ptr, (long long)(size_t)psi[0].data.ptr,
+            deferred ? (long long)(size_t)mw.ring[0].data.ptr : 0};
+  };
   // the recurrences as a WHILE node of graph g (after deps): chunks of
   // iterations until the solve is done, no host polling; returns the node
   // and the kernels of one body
@@ -353,8 +571,9 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
     const long long c0 = launch_counter();
     CPSGPU_CUDA(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
     try {
-      for (int k = 0; k < chunk; k++) iteration(0);
-      ms_loop_cond_kernel<<<1, 32, 0, s>>>(hw, st, mw.ctl.as<int>());
+      for (int k = 0; k < chunk; k++) iteration(0, deferred ? k : -1);
+      if (deferred) flush();
+      ms_loop_cond_kernel<<<1, 32, 0, s>>>(hw, st, msd, mw.ctl.as<int>());
       CPSGPU_CUDA(cudaGetLastError());
       launch_counter()++;
     } catch (...) {
@@ -409,7 +628,9 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
   const bool one_graph = (P != PREC_DOUBLE && refine);
   clk::time_point t_ref;
   if (!one_graph) {
-    iteration(1);  // the initial step of minvcg.C:140-188 (psi update from chi)
+    ensure_ring();
+    const std::vector<long long> key = graph_key();
+    iteration(1, -1);  // the initial step of minvcg.C:140-188 (psi update from chi)
     // the iterations: one graph launch, the instantiated graph kept on the
     // operator while the configuration is the same
     CachedGraph &lg = mw.loop;
@@ -465,14 +686,15 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
     cg->begin_params(a);
     cg->set_loop_limit();
     CachedGraph &fg = mw.full;
-    std::vector<long long> key2 = key;
+    ensure_ring();
+    std::vector<long long> key2 = graph_key();
     key2.push_back((long long)cg->id);
     if (fg.ge && fg.key != key2) fg.drop();
     if (!fg.ge) {
       CPSGPU_CUDA(cudaGraphCreate(&fg.g, 0));
       try {
         std::vector<cudaGraphNode_t> sinks;
-        const long long n0 = capture_segment(fg.g, nullptr, 0, sinks, [&] { iteration(1); });
+        const long long n0 = capture_segment(fg.g, nullptr, 0, sinks, [&] { iteration(1, -1); });
         long long kr = 0;
         const cudaGraphNode_t w1 = add_recurrence_loop(fg.g, sinks.data(), sinks.size(), &kr);
         cudaGraphNode_t e1;

@@ -54,6 +54,9 @@ enum ReduceOp {
 };
 
 constexpr int MS_MAX = 64;
+// iterations whose per-shift updates the multishift CG applies together
+// (multishift.cu ms_flush_kernel); the loop's chunk length
+constexpr int MS_DEFER = 8;
 
 // Device-resident scalars of the multishift CG (DiracOp::MInvCG,
 // minvcg.C:47-353), reached through SolverScalars::ext.
@@ -65,82 +68,115 @@ struct MsScalars {
   double z[2][MS_MAX], bs[MS_MAX], as[MS_MAX];
   double rsd_out[MS_MAX];
   int conv[MS_MAX], conv_prev[MS_MAX], conv_iter[MS_MAX];
+  // coefficients of the iterations since the last flush, [iteration][shift]:
+  // psi_s += hf p_s where h_upd, then p_s = hz r + ha p_s where h_adv
+  int nh;
+  double hf[MS_DEFER][MS_MAX], hz[MS_DEFER][MS_MAX], ha[MS_DEFER][MS_MAX];
+  unsigned char h_upd[MS_DEFER][MS_MAX], h_adv[MS_DEFER][MS_MAX];
 };
 
-// the shifted-system recurrences of minvcg.C, run by the last block
+// The shifted-system recurrences of minvcg.C: the shared scalars by thread 0
+// of the finalizing block, then shift s by thread s (every thread of the
+// block calls this).  One thread walking all shifts took about 1 us per
+// shift (dependent loads and FP64 divisions).
 __device__ inline void finalize_multishift(SolverScalars *st, int op, const double *sum) {
   MsScalars *ms = reinterpret_cast<MsScalars *>(st->ext);
-  const int n = ms->nshift;
+  const int n = ms->nshift, s = threadIdx.x;
+  __shared__ int go, any_running;
   if (op == RED_MS_PAP) {
-    // d = <p, (A + m_0) p>   (minvcg.C:141-148, :228-236)
-    double d = sum[0] + ms->mass[0] * sum[1];
-    ms->d = d;
-    if (!isfinite(d)) { st->done = ST_NONFINITE; return; }
-    if (d == 0.0) { st->done = ST_BREAKDOWN; return; }
-    ms->bp = ms->b;
-    ms->b = -ms->cp / d;
-    if (ms->first) {
-      // minvcg.C:152-165
-      ms->z[0][0] = ms->z[1][0] = 1.0;
-      ms->bs[0] = ms->b;
-      ms->iz = 1;
-      for (int s = 1; s < n; s++) {
-        ms->z[1 - ms->iz][s] = 1.0;
-        ms->z[ms->iz][s] = 1.0 / (1.0 - ms->b * (ms->mass[s] - ms->mass[0]));
-        ms->bs[s] = ms->b * ms->z[ms->iz][s];
-      }
-    } else {
-      // minvcg.C:238-252
-      const double b = ms->b, bp = ms->bp, a = ms->a;
-      ms->bs[0] = b;
-      ms->iz = 1 - ms->iz;
-      const int iz = ms->iz;
-      for (int s = 1; s < n; s++) {
-        if (ms->conv[s]) continue;
-        double zt = ms->z[1 - iz][s] * ms->z[iz][s] * bp /
-                    (b * a * (ms->z[iz][s] - ms->z[1 - iz][s]) +
-                     ms->z[iz][s] * bp * (1 - b * (ms->mass[s] - ms->mass[0])));
-        ms->bs[s] = b * zt / ms->z[1 - iz][s];
-        ms->z[iz][s] = zt;
+    if (s == 0) {
+      // d = <p, (A + m_0) p>   (minvcg.C:141-148, :228-236)
+      const double d = sum[0] + ms->mass[0] * sum[1];
+      ms->d = d;
+      go = 1;
+      if (!isfinite(d)) { st->done = ST_NONFINITE; go = 0; }
+      else if (d == 0.0) { st->done = ST_BREAKDOWN; go = 0; }
+      else {
+        ms->bp = ms->b;
+        ms->b = -ms->cp / d;
+        ms->iz = 1 - ms->iz;
+        if (ms->first) {
+          ms->z[0][0] = ms->z[1][0] = 1.0;
+          ms->iz = 1;
+        }
+        ms->bs[0] = ms->b;
+        st->alpha = -ms->b;  // r += b A p is r -= alpha A p
       }
     }
-    st->alpha = -ms->b;  // r += b A p is r -= alpha A p
+    __syncthreads();
+    if (!go || s == 0 || s >= n) return;
+    const double b = ms->b;
+    const int iz = ms->iz;
+    if (ms->first) {
+      // minvcg.C:152-165
+      ms->z[1 - iz][s] = 1.0;
+      ms->z[iz][s] = 1.0 / (1.0 - b * (ms->mass[s] - ms->mass[0]));
+      ms->bs[s] = b * ms->z[iz][s];
+    } else if (!ms->conv[s]) {
+      // minvcg.C:238-252
+      const double bp = ms->bp, a = ms->a;
+      const double zt = ms->z[1 - iz][s] * ms->z[iz][s] * bp /
+                        (b * a * (ms->z[iz][s] - ms->z[1 - iz][s]) +
+                         ms->z[iz][s] * bp * (1 - b * (ms->mass[s] - ms->mass[0])));
+      ms->bs[s] = b * zt / ms->z[1 - iz][s];
+      ms->z[iz][s] = zt;
+    }
     return;
   }
   // RED_MS_RR: c = |r|^2 and per-shift convergence (minvcg.C:255-304)
   const double c = sum[0];
-  ms->c = c;
-  if (!isfinite(c)) { st->done = ST_NONFINITE; return; }
-  for (int s = 0; s < n; s++) ms->conv_prev[s] = ms->conv[s];
-  if (ms->first) {
-    ms->first = 0;
-    ms->conv_all = (c < ms->rsd_sq[0]) ? 1 : 0;
-  } else {
-    ms->k += 1;
-    const int iz = ms->iz;
-    for (int s = 0; s < n; s++) {
-      if (ms->conv[s]) continue;
-      double css = c * ms->z[iz][s] * ms->z[iz][s];
+  const bool first = ms->first;  // read by every thread before thread 0 clears it
+  __syncthreads();
+  if (s == 0) {
+    ms->c = c;
+    go = isfinite(c) ? 1 : 0;
+    if (!go) st->done = ST_NONFINITE;
+    any_running = 0;
+    if (first) ms->first = 0;
+    else if (go) ms->k += 1;
+  }
+  __syncthreads();
+  if (!go) return;
+  const int iz = ms->iz;
+  const bool was = s < n && ms->conv[s];
+  bool conv = was;
+  if (s < n) {
+    ms->conv_prev[s] = was;
+    if (!first && !was) {
+      const double css = c * ms->z[iz][s] * ms->z[iz][s];
       if (css < ms->rsd_sq[s]) {
+        conv = true;
         ms->conv[s] = 1;
         ms->rsd_out[s] = css;
         ms->conv_iter[s] = ms->k;
       }
     }
-    int all = ms->conv[0];
-    if (all)
-      for (int s = 0; s < n; s++)
-        if (!ms->conv[s]) all = 0;
-    ms->conv_all = all;
+    if (!conv) any_running = 1;
   }
-  if (ms->conv_all) st->done = ST_CONVERGED;
-  else if (ms->k >= ms->max_iter) st->done = ST_MAX_ITER;
-  // coefficients of the next direction update (minvcg.C:204-225)
-  ms->a = c / ms->cp;
-  const int iz = ms->iz;
-  for (int s = 1; s < n; s++)
-    if (!ms->conv[s]) ms->as[s] = ms->a * (ms->z[iz][s] * ms->bs[s]) / (ms->z[1 - iz][s] * ms->b);
-  ms->cp = c;
+  __syncthreads();
+  if (s == 0) {
+    ms->conv_all = first ? ((c < ms->rsd_sq[0]) ? 1 : 0) : !any_running;
+    if (ms->conv_all) st->done = ST_CONVERGED;
+    else if (ms->k >= ms->max_iter) st->done = ST_MAX_ITER;
+    ms->a = c / ms->cp;
+    ms->cp = c;
+  }
+  __syncthreads();
+  // coefficients of this iteration's updates and of the next direction (minvcg.C:204-225)
+  const int j = ms->nh;
+  if (s < n) {
+    const double a = ms->a;
+    if (s > 0 && !conv) ms->as[s] = a * (ms->z[iz][s] * ms->bs[s]) / (ms->z[1 - iz][s] * ms->b);
+    if (j < MS_DEFER) {
+      ms->hf[j][s] = -ms->bs[s] * ms->weight[s];
+      ms->hz[j][s] = (s == 0) ? 1.0 : ms->z[iz][s];
+      ms->ha[j][s] = (s == 0) ? a : ms->as[s];
+      ms->h_upd[j][s] = !was;
+      ms->h_adv[j][s] = (st->done == 0) && !conv;
+    }
+  }
+  __syncthreads();
+  if (s == 0) ms->nh = j + 1;
 }
 
 __device__ __forceinline__ bool finite_d(double x) { return isfinite(x); }
@@ -198,11 +234,7 @@ __device__ inline void finalize_scalars(SolverScalars *st, int op, const double 
       else if (sum[0] <= st->stop || st->max_iter <= 0) st->done = ST_CONVERGED;
       break;
     }
-    case RED_MS_PAP:
-    case RED_MS_RR:
-      finalize_multishift(st, op, sum);
-      break;
-    default:
+    default:  // RED_STORE; the multishift operations follow in finalize_multishift
       break;
   }
 }
@@ -296,6 +328,10 @@ __global__ void __launch_bounds__(FINALIZE_THREADS)
     for (int k = 0; k < NV; k++)
       for (int w = 0; w < FINALIZE_THREADS / 32; w++) tot[k] += sm[w][k];
     finalize_scalars(&st[solve], op, tot);
+  }
+  if (op == RED_MS_PAP || op == RED_MS_RR) {
+    __syncthreads();
+    finalize_multishift(&st[solve], op, st[solve].sum);
   }
 }
 
