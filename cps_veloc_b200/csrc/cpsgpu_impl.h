@@ -235,6 +235,7 @@ struct HopLaunch {
   const void *halo_fwd = nullptr, *halo_bwd = nullptr;  // t halos of a decomposed lattice (dd.cu)
   int sub = 0;  // HopSub: all sites, or (decomposed lattice) the interior or the two t-end slices
   double *partials = nullptr;  // the reduction's per-block partials (null: the lattice's buffer)
+  cudaGraphConditionalHandle *cond = nullptr;  // set by the finalize: this iteration's reliable update (one solve)
 };
 void launch_hop(const Dirac &D, const HopLaunch &L, const SpinorView &in, const SpinorView &out,
                 const SpinorView &x, const SpinorView &r, const SpinorView &sol, const SpinorView &p,
@@ -290,7 +291,7 @@ void launch_norm(cudaStream_t s, int prec, const SpinorView &f, SolverScalars *s
 // sum the per-block partials (nv values each, nblk blocks per solve) of the
 // preceding reducing kernel and update each solve's scalars with op
 void launch_finalize(cudaStream_t s, int nv, const double *partials, SolverScalars *st, int op, unsigned nblk,
-                     int nsolves, int gate);
+                     int nsolves, int gate, const cudaGraphConditionalHandle *cond = nullptr);
 // st[k] <- value (host-side init through a kernel so graphs can replay it)
 void launch_init_scalars(cudaStream_t s, SolverScalars *st, int nrhs, const SolverScalars &init);
 

@@ -150,7 +150,7 @@ void hop(const Dirac &D, int ep, int cb, int dag, int norm, const SpinorView &in
   pick(recon, ep, dag)<<<grid, block, 0, lat.stream>>>(hp, v, st, partials);
   CPSGPU_CUDA(cudaGetLastError());
   if (norm) {  // sum the per-block partials of |out|^2, |x|^2 into st->sum
-    finalize_kernel<2><<<1, FINALIZE_THREADS, 0, lat.stream>>>(partials, st, RED_STORE, grid.x, GATE_NONE);
+    finalize_kernel<2><<<1, finalize_threads(grid.x, RED_STORE), 0, lat.stream>>>(partials, st, RED_STORE, grid.x, GATE_NONE);
     CPSGPU_CUDA(cudaGetLastError());
   }
 }

@@ -288,15 +288,23 @@ constexpr int FINALIZE_THREADS = 1024;
 // One block per solve: sum its nblk partials (thread-strided, then the warp
 // and block trees, always in the same order) and finalize its scalars.  The
 // gate is the one the reducing kernel had, so a solve it skipped is skipped
-// here too.
+// here too.  The block has the warps that nblk partials fill, at most
+// FINALIZE_THREADS threads (the stride, so the order of the sum does not
+// depend on it): a small solve's one step from the next kernel is this
+// kernel's latency.  set_cond: cond is the condition of this iteration's
+// reliable update (one solve), set here instead of by a kernel of its own.
 template <int NV>
 __global__ void __launch_bounds__(FINALIZE_THREADS)
-    finalize_kernel(const double *partials, SolverScalars *st, int op, unsigned nblk, int gate) {
+    finalize_kernel(const double *partials, SolverScalars *st, int op, unsigned nblk, int gate,
+                    cudaGraphConditionalHandle cond = 0, int set_cond = 0) {
   const unsigned solve = blockIdx.x;
-  if (gate == 1 && st[solve].done) return;                              // GATE_RUNNING
-  if (gate == 2 && (st[solve].done || !st[solve].reliable)) return;     // GATE_RELIABLE
-  __shared__ double sm[FINALIZE_THREADS / 32][NV];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if ((gate == 1 && st[solve].done) ||                              // GATE_RUNNING
+      (gate == 2 && (st[solve].done || !st[solve].reliable))) {     // GATE_RELIABLE
+    if (tid == 0 && set_cond) cudaGraphSetConditional(cond, 0);
+    return;
+  }
+  __shared__ double sm[FINALIZE_THREADS / 32][NV];
   const double *part = partials + (size_t)solve * nblk * NV;
   double acc[NV];
 #pragma unroll
@@ -325,14 +333,24 @@ __global__ void __launch_bounds__(FINALIZE_THREADS)
   __syncthreads();
   if (tid == 0) {
     double tot[4] = {0, 0, 0, 0};
+    const int nwarp = (int)(blockDim.x >> 5);
     for (int k = 0; k < NV; k++)
-      for (int w = 0; w < FINALIZE_THREADS / 32; w++) tot[k] += sm[w][k];
+      for (int w = 0; w < nwarp; w++) tot[k] += sm[w][k];
     finalize_scalars(&st[solve], op, tot);
+    if (set_cond) cudaGraphSetConditional(cond, (!st[solve].done && st[solve].reliable) ? 1u : 0u);
   }
   if (op == RED_MS_PAP || op == RED_MS_RR) {
     __syncthreads();
     finalize_multishift(&st[solve], op, st[solve].sum);
   }
+}
+
+// threads of a finalize launch over nblk partials (the multishift operations
+// need one per shift)
+inline unsigned finalize_threads(unsigned nblk, int op) {
+  unsigned t = (nblk + 31u) & ~31u;
+  if ((op == RED_MS_PAP || op == RED_MS_RR) && t < (unsigned)MS_MAX) t = MS_MAX;
+  return t > FINALIZE_THREADS ? FINALIZE_THREADS : t;
 }
 
 }  // namespace cpsgpu

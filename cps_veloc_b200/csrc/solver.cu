@@ -109,9 +109,11 @@ CgSolver::~CgSolver() {
 // Emit out-of-place MatPcDagMatPc on `in` with a final epilogue.
 //   final == EP_CG: r -= alpha A in; sol += alpha in; RED_CG_RR
 //   final == EP_RES: r_out = b - A in; reduce with red_op
-// The M half reduces |M in|^2 (RED_PAP) when pap is set.
+// The M half reduces |M in|^2 (RED_PAP) when pap is set.  cond: the condition
+// of the iteration's reliable update, set by the last finalize.
 void CgSolver::emit_mdagm(int prec, const SpinorView &in, OpWork &w, int final_ep, int pap, int red_op, int gate,
-                          const SpinorView &rv, int pr, const SpinorView &solv, int px) {
+                          const SpinorView &rv, int pr, const SpinorView &solv, int px,
+                          cudaGraphConditionalHandle *cond) {
   SolverScalars *stp = st.as<SolverScalars>();
   const bool mob = (D.kind == KIND_MOBIUS);
   HopLaunch Lh;
@@ -163,6 +165,7 @@ void CgSolver::emit_mdagm(int prec, const SpinorView &in, OpWork &w, int final_e
   Lh.red_op = red_op;
   Lh.pr = pr;
   Lh.px = px;
+  Lh.cond = cond;
   if (final_ep == EP_CG) {
     Lh.ep = mix_last ? EP_MIX_CG : EP_CG;
     launch_hop(D, Lh, hop_in, none(), x, rv, solv, in, none(), stp);
@@ -188,25 +191,32 @@ void CgSolver::emit_reliable_update() {
 // launch its FP64 operator's grids at all.
 void CgSolver::emit_iteration(bool conditional) {
   Lattice &L = *D.lat;
-  const int px = (sloppy == PREC_DOUBLE) ? PREC_DOUBLE : PREC_SINGLE;
+  const int px = px_of(sloppy);
   SolverScalars *stp = st.as<SolverScalars>();
   const SpinorView solv = (sloppy == PREC_DOUBLE) ? x64.view() : xs.view();
-  emit_mdagm(sloppy, p.view(), ws, EP_CG, 1, RED_CG_RR, GATE_RUNNING, r.view(), sloppy, solv, px);
+  const cudaStream_t s = L.stream;
+  cudaStreamCaptureStatus cs;
+  cudaGraph_t g = nullptr;
+  const cudaGraphNode_t *deps = nullptr;
+  size_t nd = 0;
+  cudaGraphConditionalHandle h = 0;
+  if (conditional && sloppy != PREC_DOUBLE) {
+    CPSGPU_CUDA(cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, &nd));
+    CPSGPU_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
+  }
+  // one solve: its finalize sets the condition; several: a kernel looks at all of them
+  const bool cond_in_finalize = g && nrhs == 1;
+  emit_mdagm(sloppy, p.view(), ws, EP_CG, 1, RED_CG_RR, GATE_RUNNING, r.view(), sloppy, solv, px,
+             cond_in_finalize ? &h : nullptr);
   if (sloppy != PREC_DOUBLE) {
     if (!conditional) {
       emit_reliable_update();
     } else {
-      const cudaStream_t s = L.stream;
-      cudaStreamCaptureStatus cs;
-      cudaGraph_t g;
-      const cudaGraphNode_t *deps = nullptr;
-      size_t nd = 0;
-      CPSGPU_CUDA(cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, &nd));
-      cudaGraphConditionalHandle h;
-      CPSGPU_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
-      reliable_cond_kernel<<<1, 32, 0, s>>>(h, stp, nrhs);
-      CPSGPU_CUDA(cudaGetLastError());
-      launch_counter()++;
+      if (!cond_in_finalize) {
+        reliable_cond_kernel<<<1, 32, 0, s>>>(h, stp, nrhs);
+        CPSGPU_CUDA(cudaGetLastError());
+        launch_counter()++;
+      }
       CPSGPU_CUDA(cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, &nd));
       cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
       cp.conditional.handle = h;

@@ -81,7 +81,8 @@ struct CgSolver {
   void emit_iteration(bool conditional = false);
   void emit_reliable_update();
   void emit_mdagm(int prec, const SpinorView &in, OpWork &w, int final_ep, int pap, int red_op, int gate,
-                  const SpinorView &rv, int pr, const SpinorView &solv, int px);
+                  const SpinorView &rv, int pr, const SpinorView &solv, int px,
+                  cudaGraphConditionalHandle *cond = nullptr);
 };
 
 // Independent solves in one graph launch (solver.cu); each solver set up for
