@@ -1615,7 +1615,7 @@ int cpsgpu_set_hop_shape(cpsgpu_dirac d, int prec, int sites, int slices, int sl
     const dim3 b((unsigned)sites, (unsigned)slices, (unsigned)slices_per_thread);
     const int eps[] = {EP_STORE, EP_AXPY, EP_CG, EP_RES};
     CPSGPU_CUDA(cudaStreamSynchronize(D.lat->stream));
-    for (int ep : eps) tune_set(TuneKey{prec, D.lat->recon(prec), ep, D.kind, D.ls}, b, order);
+    for (int ep : eps) tune_set(TuneKey{prec, D.lat->recon(prec), ep, D.kind, D.ls}, b, order, true);
     // captured graphs hold the launches of the old shape
     drop_captured(d);
     return CPSGPU_OK;

@@ -263,6 +263,11 @@ __device__ __forceinline__ void acc2_store(const acc2 &a, float *acc) {
 // The accumulator of one hop site: the scalar form for FP64, the packed
 // form for FP32 arithmetic (FP32 and FP16 storage).
 template <typename R> struct HopAcc {
+  using Half = half_spinor<R>;  // a link times a half spinor
+  static __device__ __forceinline__ Half mul(const su3<R> &u, const half_spinor<R> &h, bool dagger) {
+    return link_mul(u, h, dagger);
+  }
+  static __device__ __forceinline__ Half pack(const half_spinor<R> &h) { return h; }
   R a[24];
   __device__ __forceinline__ void zero() {
 #pragma unroll
@@ -273,22 +278,25 @@ template <typename R> struct HopAcc {
     reconstruct_acc(a, link_mul(u, h, dagger), mu, k, w);
   }
   // += w * reconstruct(g)
-  __device__ __forceinline__ void add(const half_spinor<R> &g, int mu, R k, R w) { reconstruct_acc(a, g, mu, k, w); }
+  __device__ __forceinline__ void add(const Half &g, int mu, R k, R w) { reconstruct_acc(a, g, mu, k, w); }
   __device__ __forceinline__ void store(R *acc) const {
 #pragma unroll
     for (int k = 0; k < 24; k++) acc[k] = a[k];
   }
 };
 template <> struct HopAcc<float> {
+  using Half = hs2;
+  static __device__ __forceinline__ Half mul(const su3<float> &u, const half_spinor<float> &h, bool dagger) {
+    return link_mul2(u, pack_hs2(h), dagger);
+  }
+  static __device__ __forceinline__ Half pack(const half_spinor<float> &h) { return pack_hs2(h); }
   acc2 a;
   __device__ __forceinline__ void zero() { acc2_zero(a); }
   __device__ __forceinline__ void hop(const su3<float> &u, const half_spinor<float> &h, bool dagger, int mu, float k,
                                       float w) {
     reconstruct_acc2(a, link_mul2(u, pack_hs2(h), dagger), mu, k, w);
   }
-  __device__ __forceinline__ void add(const half_spinor<float> &g, int mu, float k, float w) {
-    reconstruct_acc2(a, pack_hs2(g), mu, k, w);
-  }
+  __device__ __forceinline__ void add(const Half &g, int mu, float k, float w) { reconstruct_acc2(a, g, mu, k, w); }
   __device__ __forceinline__ void store(float *acc) const { acc2_store(a, acc); }
 };
 

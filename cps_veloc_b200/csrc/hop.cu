@@ -15,6 +15,14 @@ HopFn pick(int prec, const HopSel &q) {
   return prec == PREC_DOUBLE ? pick_hop_double(q) : prec == PREC_SINGLE ? pick_hop_single(q) : pick_hop_half(q);
 }
 
+// Launches of at most this many 5D sites (right-hand sides included) run four
+// threads per site (hop_split_kernel).  Microseconds per CG iteration without
+// / with, by sites: FP64 256 (Wilson 4^3x8) 41.7 / 28.1, 4096 (8^3x16) 40.9 /
+// 29.5, 16384 (DWF 8^4 Ls=8) 46.7 / 48.9, 32768 52.7 / 64.7; FP32 inner
+// solve 256 42.7 / 34.3, 16384 44.5 / 37.9, 32768 45.1 / 49.1; 8 right-hand
+// sides of 2048 sites FP64 46.8 / 48.6, FP32 48.6 / 40.5
+constexpr long split_sites(int prec) { return prec == PREC_DOUBLE ? 8192 : 16384; }
+
 size_t real_size(int prec) { return prec == PREC_DOUBLE ? 8 : 4; }
 
 }  // namespace
@@ -78,7 +86,9 @@ void launch_hop(const Dirac &D, const HopLaunch &L, const SpinorView &in, const 
   // block.z of a tuned shape: slices per thread (2: DWF slice pairs)
   const int ns = (block.z == 2 && hp.dwf && !mix && !halo && L.prec != PREC_DOUBLE && D.ls % (4 * (int)block.y) == 0) ? 2 : 1;
   block.z = 1;
-  HopFn fn = pick(L.prec, HopSel{recon, L.ep, L.pr, L.px, L.dag != 0, ns, halo});
+  const bool split_mu = !mix && !split && lat.vh * D.ls * in.nrhs <= split_sites(L.prec) && !hop_forced(key);
+  if (split_mu) block = dim3(SPLIT_BX, 1, 4);
+  HopFn fn = pick(L.prec, HopSel{recon, L.ep, L.pr, L.px, L.dag != 0, ns, halo, split_mu});
   unsigned nsb;
   if (L.sub == SUB_BOUNDARY) {
     hp.subn = (hp.face + (int)block.x - 1) / (int)block.x;
@@ -93,9 +103,9 @@ void launch_hop(const Dirac &D, const HopLaunch &L, const SpinorView &in, const 
     hp.i0 = (L.sub == SUB_INTERIOR) ? hp.face : 0;
     hp.iend = hp.i0 + (int)nsites;
   }
-  hp.nsg = ns == 2 ? D.ls / (2 * (int)block.y) : (D.ls + block.y - 1) / block.y;
+  hp.nsg = (ns == 2 && !split_mu) ? D.ls / (2 * (int)block.y) : (D.ls + block.y - 1) / block.y;
   // ORDER_SITES: the slice groups on the grid's y (blocks run x fastest)
-  const bool sites_first = (hop_order(key) == ORDER_SITES && hp.nsg > 1);
+  const bool sites_first = (hop_order(key) == ORDER_SITES && hp.nsg > 1 && !split_mu);
   hp.spar = (hp.dwf && !mix && block.y > 1 && D.ls % (2 * block.y) == 0) ? 1 : 0;
   hp.nrhs = in.nrhs;
   hp.rtile = std::max(1, std::min(D.rhs_tile(L.prec, in.nrhs), in.nrhs));

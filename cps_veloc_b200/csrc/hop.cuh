@@ -134,74 +134,111 @@ __device__ __forceinline__ half_spinor<R> load_halo(const void *p, int face, lon
   return r;
 }
 
-// acc = sum over mu of the forward and backward hops into output site i,
-// slice sl, whose 4D parity is pout (input parity pin = 1 - pout).
-// All site arithmetic is 32-bit; the coordinates come from three
-// multiply-high divisions and each neighbour index from i by a stride.
+// Coordinates of output site i on 4D parity pout: all site arithmetic is
+// 32-bit; the coordinates come from three multiply-high divisions and each
+// neighbour index from i by a stride.
+struct HopSite {
+  int i, xh, x, c[4], stride[4];
+  __device__ __forceinline__ HopSite(const HopParams &hp, int i_, int pout) : i(i_) {
+    const int hx = hp.hx, Ly = hp.L[1], Lz = hp.L[2];
+    const int q1 = hp.dhx.div(i);
+    xh = i - q1 * hx;
+    const int q2 = hp.dly.div(q1);
+    const int y = q1 - q2 * Ly;
+    const int t = hp.dlz.div(q2);
+    const int z = q2 - t * Lz;
+    x = 2 * xh + ((y + z + t + pout) & 1);
+    c[0] = x;
+    c[1] = y;
+    c[2] = z;
+    c[3] = t;
+    stride[0] = 0;
+    stride[1] = hx;
+    stride[2] = hx * Ly;
+    stride[3] = hx * Ly * Lz;
+  }
+};
+
+// One hop of direction mu (a compile-time constant once inlined) into the
+// site, slice sl: its half spinor g, to be accumulated with the weight w (the
+// storage scale and the boundary sign ride on the accumulating FMAs).
 // HALO: the t hops across a slab's ends read the halos (t-slab decomposition);
 // a separate instantiation, so the undecomposed kernels carry none of it.
+template <int P, int RECON, bool DAG, bool HALO, bool FWD>
+__device__ __forceinline__ void hop_dir(const HopParams &hp, const HopViews &v, const Slice<P> &in, const HopSite &q,
+                                        int mu, long sl, int pout,
+                                        typename HopAcc<typename PrecTraits<P>::real>::Half &g,
+                                        typename PrecTraits<P>::real &w) {
+  using R = typename PrecTraits<P>::real;
+  using A = HopAcc<R>;
+  const int pin = 1 - pout, i = q.i;
+  // sdag is a compile-time +-1, so every (1 -+ gamma) sign folds into adds
+  constexpr R sdag = DAG ? R(-1) : R(1);
+  if constexpr (FWD) {  // U_mu(x) (1 - sdag g_mu) psi(x + mu)
+    const bool wrap = (q.c[mu] == hp.L[mu] - 1);
+    int j;
+    if (mu == 0) j = i - q.xh + ((wrap ? 0 : q.x + 1) >> 1);
+    else j = wrap ? i - (hp.L[mu] - 1) * q.stride[mu] : i + q.stride[mu];
+    if (HALO && mu == 3 && wrap) {
+      // x + t lives on the next slab, which sent its projected half spinor
+      su3<R> u;
+      LinkIO<P, RECON>::load(v.U, pout, mu, i, u);
+      g = A::mul(u, load_halo<R>(v.hf, hp.face, sl, j), false);
+      w = (hp.tb_fwd && hp.bc[mu] < 0) ? R(-1) : R(1);
+    } else {
+      R psi[24], sc;
+      in.load_raw(j, psi, sc);
+      su3<R> u;
+      LinkIO<P, RECON>::load(v.U, pout, mu, i, u);
+      g = A::mul(u, project(psi, mu, -sdag), false);
+      w = (wrap && hp.bc[mu] < 0 && (!HALO || mu != 3 || hp.tb_fwd)) ? -sc : sc;
+    }
+  } else {  // U_mu(x - mu)^dagger (1 + sdag g_mu) psi(x - mu)
+    const bool wrap = (q.c[mu] == 0);
+    int j;
+    if (mu == 0) j = i - q.xh + ((wrap ? hp.L[0] - 1 : q.x - 1) >> 1);
+    else j = wrap ? i + (hp.L[mu] - 1) * q.stride[mu] : i - q.stride[mu];
+    if (HALO && mu == 3 && wrap) {
+      // x - t and its link live on the previous slab, which sent U^dagger (1 + sdag g_t) psi
+      g = A::pack(load_halo<R>(v.hb, hp.face, sl, i));
+      w = (hp.tb_bwd && hp.bc[mu] < 0) ? R(-1) : R(1);
+    } else {
+      R psi[24], sc;
+      in.load_raw(j, psi, sc);
+      su3<R> u;
+      LinkIO<P, RECON>::load(v.U, pin, mu, j, u);
+      g = A::mul(u, project(psi, mu, sdag), true);
+      w = (wrap && hp.bc[mu] < 0 && (!HALO || mu != 3 || hp.tb_bwd)) ? -sc : sc;
+    }
+  }
+}
+
+// A += both hops of direction mu
+template <int P, int RECON, bool DAG, bool HALO>
+__device__ __forceinline__ void hop_mu(const HopParams &hp, const HopViews &v, const Slice<P> &in, const HopSite &q,
+                                       int mu, long sl, int pout, HopAcc<typename PrecTraits<P>::real> &A) {
+  using R = typename PrecTraits<P>::real;
+  constexpr R sdag = DAG ? R(-1) : R(1);
+  typename HopAcc<R>::Half g;
+  R w;
+  hop_dir<P, RECON, DAG, HALO, true>(hp, v, in, q, mu, sl, pout, g, w);
+  A.add(g, mu, -sdag, w);
+  hop_dir<P, RECON, DAG, HALO, false>(hp, v, in, q, mu, sl, pout, g, w);
+  A.add(g, mu, sdag, w);
+}
+
+// acc = sum over mu of the forward and backward hops into output site i,
+// slice sl, whose 4D parity is pout (input parity 1 - pout).
 template <int P, int RECON, bool DAG, bool HALO>
 __device__ __forceinline__ void hop_site(const HopParams &hp, const HopViews &v, int i, long sl,
                                          int pout, typename PrecTraits<P>::real *acc) {
-  using R = typename PrecTraits<P>::real;
-  const int pin = 1 - pout;
-  const int hx = hp.hx, Ly = hp.L[1], Lz = hp.L[2];
-  const int q1 = hp.dhx.div(i);
-  const int xh = i - q1 * hx;
-  const int q2 = hp.dly.div(q1);
-  const int y = q1 - q2 * Ly;
-  const int t = hp.dlz.div(q2);
-  const int z = q2 - t * Lz;
-  const int x = 2 * xh + ((y + z + t + pout) & 1);
-  const int c[4] = {x, y, z, t};
-  const int stride[4] = {0, hx, hx * Ly, hx * Ly * Lz};
+  const HopSite q(hp, i, pout);
   const Slice<P> in(v.in, sl);
-  // sdag is a compile-time +-1, so every (1 -+ gamma) sign folds into adds
-  constexpr R sdag = DAG ? R(-1) : R(1);
-  HopAcc<R> A;
+  HopAcc<typename PrecTraits<P>::real> A;
   A.zero();
 #pragma unroll
-  for (int mu = 0; mu < 4; mu++) {
-    // forward: U_mu(x) (1 - sdag g_mu) psi(x + mu)
-    {
-      const bool wrap = (c[mu] == hp.L[mu] - 1);
-      int j;
-      if (mu == 0) j = i - xh + ((wrap ? 0 : x + 1) >> 1);
-      else j = wrap ? i - (hp.L[mu] - 1) * stride[mu] : i + stride[mu];
-      if (HALO && mu == 3 && wrap) {
-        // x + t lives on the next slab, which sent its projected half spinor
-        su3<R> u;
-        LinkIO<P, RECON>::load(v.U, pout, mu, i, u);
-        A.hop(u, load_halo<R>(v.hf, hp.face, sl, j), false, mu, -sdag, (hp.tb_fwd && hp.bc[mu] < 0) ? R(-1) : R(1));
-      } else {
-        R psi[24], sc;
-        in.load_raw(j, psi, sc);
-        su3<R> u;
-        LinkIO<P, RECON>::load(v.U, pout, mu, i, u);
-        // the storage scale and the boundary sign ride on the accumulating FMAs
-        A.hop(u, project(psi, mu, -sdag), false, mu, -sdag,
-              (wrap && hp.bc[mu] < 0 && (!HALO || mu != 3 || hp.tb_fwd)) ? -sc : sc);
-      }
-    }
-    // backward: U_mu(x - mu)^dagger (1 + sdag g_mu) psi(x - mu)
-    {
-      const bool wrap = (c[mu] == 0);
-      int j;
-      if (mu == 0) j = i - xh + ((wrap ? hp.L[0] - 1 : x - 1) >> 1);
-      else j = wrap ? i + (hp.L[mu] - 1) * stride[mu] : i - stride[mu];
-      if (HALO && mu == 3 && wrap) {
-        // x - t and its link live on the previous slab, which sent U^dagger (1 + sdag g_t) psi
-        A.add(load_halo<R>(v.hb, hp.face, sl, i), mu, sdag, (hp.tb_bwd && hp.bc[mu] < 0) ? R(-1) : R(1));
-      } else {
-        R psi[24], sc;
-        in.load_raw(j, psi, sc);
-        su3<R> u;
-        LinkIO<P, RECON>::load(v.U, pin, mu, j, u);
-        A.hop(u, project(psi, mu, sdag), true, mu, sdag,
-              (wrap && hp.bc[mu] < 0 && (!HALO || mu != 3 || hp.tb_bwd)) ? -sc : sc);
-      }
-    }
-  }
+  for (int mu = 0; mu < 4; mu++)
+    hop_mu<P, RECON, DAG, HALO>(hp, v, in, q, mu, sl, pout, A);
   A.store(acc);
 }
 
@@ -214,16 +251,9 @@ __device__ __forceinline__ void hop_site2(const HopParams &hp, const HopViews &v
                                           typename PrecTraits<P>::real *acc1) {
   using R = typename PrecTraits<P>::real;
   const int pin = 1 - pout;
-  const int hx = hp.hx, Ly = hp.L[1], Lz = hp.L[2];
-  const int q1 = hp.dhx.div(i);
-  const int xh = i - q1 * hx;
-  const int q2 = hp.dly.div(q1);
-  const int y = q1 - q2 * Ly;
-  const int t = hp.dlz.div(q2);
-  const int z = q2 - t * Lz;
-  const int x = 2 * xh + ((y + z + t + pout) & 1);
-  const int c[4] = {x, y, z, t};
-  const int stride[4] = {0, hx, hx * Ly, hx * Ly * Lz};
+  const HopSite q(hp, i, pout);
+  const int xh = q.xh, x = q.x;
+  const int (&c)[4] = q.c, (&stride)[4] = q.stride;
   const Slice<P> in0(v.in, sl0), in1(v.in, sl1);
   constexpr R sdag = DAG ? R(-1) : R(1);
   HopAcc<R> A0, A1;
@@ -264,17 +294,19 @@ __device__ __forceinline__ void hop_site2(const HopParams &hp, const HopViews &v
   A1.store(acc1);
 }
 
-// Fifth-direction hop of the Shamir DWF operator, accumulated into acc.
+// Fifth-direction hop of the Shamir DWF operator: the stored halves q, w of
+// the neighbouring slices and their weights
 template <int P, bool DAG>
-__device__ __forceinline__ void hop5_dwf(const HopParams &hp, const HopViews &v, int i, int s, long rhs,
-                                         typename PrecTraits<P>::real *acc) {
+__device__ __forceinline__ void hop5_load(const HopParams &hp, const HopViews &v, int i, int s, long rhs,
+                                          typename PrecTraits<P>::real *q, typename PrecTraits<P>::real *w,
+                                          typename PrecTraits<P>::real &wq, typename PrecTraits<P>::real &ww) {
   using R = typename PrecTraits<P>::real;
   const int ls = hp.ls;
   // the half fed from s-1 is the upper one for D, the lower one for D^dagger
   // (register arrays are only ever indexed with compile-time offsets)
   const int sb = (s == 0) ? ls - 1 : s - 1, sa = (s == ls - 1) ? 0 : s + 1;
   const R wb = R((s == 0) ? hp.h5wall : hp.h5), wa = R((s == ls - 1) ? hp.h5wall : hp.h5);
-  R q[12], w[12], sq_, sw_;
+  R sq_, sw_;
   if constexpr (!DAG) {
     Slice<P>(v.in, rhs * ls + sb).load_half_raw(i, 0, q, sq_);
     Slice<P>(v.in, rhs * ls + sa).load_half_raw(i, 1, w, sw_);
@@ -282,7 +314,17 @@ __device__ __forceinline__ void hop5_dwf(const HopParams &hp, const HopViews &v,
     Slice<P>(v.in, rhs * ls + sa).load_half_raw(i, 0, q, sq_);
     Slice<P>(v.in, rhs * ls + sb).load_half_raw(i, 1, w, sw_);
   }
-  const R wq = (DAG ? wa : wb) * sq_, ww = (DAG ? wb : wa) * sw_;
+  wq = (DAG ? wa : wb) * sq_;
+  ww = (DAG ? wb : wa) * sw_;
+}
+
+// ... accumulated into acc
+template <int P, bool DAG>
+__device__ __forceinline__ void hop5_dwf(const HopParams &hp, const HopViews &v, int i, int s, long rhs,
+                                         typename PrecTraits<P>::real *acc) {
+  using R = typename PrecTraits<P>::real;
+  R q[12], w[12], wq, ww;
+  hop5_load<P, DAG>(hp, v, i, s, rhs, q, w, wq, ww);
 #pragma unroll
   for (int k = 0; k < 12; k++) {
     acc[k] += wq * q[k];
@@ -603,6 +645,140 @@ __global__ void __launch_bounds__(256, (hop_min_blocks<P, NS>())) hop_kernel(con
   hop_epilogue<P, EP, PR, PX>(hp, v, st, rhs, sl, s, i, active, acc, red);
   if constexpr (NV > 0) {
     if (!ep_axpy(EP) || hp.norm) block_partial<NV>(reinterpret_cast<double(&)[NV]>(red), partials, (unsigned)rhs, (unsigned)sb, nblk);
+  }
+}
+
+// ---- the hop of a small lattice: four threads per output site
+// A lattice that does not fill the GPU runs at the latency of one thread's
+// chain of eight directions.  Here thread z of a site computes the two half
+// spinors U h of direction mu = z (z = 3 also fetches the fifth direction's
+// operands), and thread z = 0 accumulates all of them from shared memory in
+// hop_site's order and applies the epilogue: a quarter of the chain, four
+// times the warps, the same bits.  A block is 32 sites of one slice (a warp
+// per direction, so mu is uniform).  Wilson and DWF, no halos, no mixing; the
+// rule is at split_sites in hop.cu.
+constexpr int SPLIT_BX = 32;
+
+// the two half spinors of one direction and their weights in shared memory
+template <typename R> struct SplitSlot {
+  R v[26][SPLIT_BX];
+  __device__ __forceinline__ void put(const R *a, const R *b, R wa, R wb, int x) {
+#pragma unroll
+    for (int k = 0; k < 12; k++) {
+      v[k][x] = a[k];
+      v[12 + k][x] = b[k];
+    }
+    v[24][x] = wa;
+    v[25][x] = wb;
+  }
+  __device__ __forceinline__ void get(R *a, R *b, R &wa, R &wb, int x) const {
+#pragma unroll
+    for (int k = 0; k < 12; k++) {
+      a[k] = v[k][x];
+      b[k] = v[12 + k][x];
+    }
+    wa = v[24][x];
+    wb = v[25][x];
+  }
+};
+template <typename H, typename R> __device__ __forceinline__ void half_reals(const H &h, R *a) {
+  static_assert(sizeof(H) == 12 * sizeof(R), "a half spinor is 12 reals");
+  const R *p = reinterpret_cast<const R *>(&h);
+#pragma unroll
+  for (int k = 0; k < 12; k++) a[k] = p[k];
+}
+template <typename H, typename R> __device__ __forceinline__ void reals_half(const R *a, H &h) {
+  R *p = reinterpret_cast<R *>(&h);
+#pragma unroll
+  for (int k = 0; k < 12; k++) p[k] = a[k];
+}
+
+template <int P, int RECON, int EP, int PR, int PX, bool DAG>
+__global__ void __launch_bounds__(4 * SPLIT_BX) hop_split_kernel(const HopParams hp, const HopViews v,
+                                                                 SolverScalars *st, double *partials) {
+  using R = typename PrecTraits<P>::real;
+  using A = HopAcc<R>;
+  static_assert(!ep_mix(EP), "no mixing epilogues");
+  constexpr R sdag = DAG ? R(-1) : R(1);
+  // blockIdx.x = (site block, slice, rhs within the tile), rhs fastest
+  const int rin = blockIdx.x % hp.rtile, sb = blockIdx.x / hp.rtile;
+  const long rhs = (long)blockIdx.z * hp.rtile + rin;
+  if (rhs >= hp.nrhs) return;
+  if (hp.gate == GATE_RUNNING && st[rhs].done) return;
+  if (hp.gate == GATE_RELIABLE && (st[rhs].done || !st[rhs].reliable)) return;
+  const unsigned nblk = gridDim.x / hp.rtile;
+  const int s = sb % hp.ls, z = threadIdx.z, x = threadIdx.x;
+  const int i = (sb / hp.ls) * SPLIT_BX + x;
+  const bool active = i < hp.vh;
+  const long sl = rhs * hp.ls + s;
+  const int pin = hp.dwf ? ((s + hp.cb) & 1) : hp.cb, pout = 1 - pin;
+  __shared__ SplitSlot<R> slot[4];  // mu = 1, 2, 3 and the fifth direction
+  typename A::Half gf, gb;
+  R wf, wb;
+  if (active) {
+    const HopSite q(hp, i, pout);
+    const Slice<P> in(v.in, sl);
+    auto both = [&](int mu) {
+      hop_dir<P, RECON, DAG, false, true>(hp, v, in, q, mu, sl, pout, gf, wf);
+      hop_dir<P, RECON, DAG, false, false>(hp, v, in, q, mu, sl, pout, gb, wb);
+    };
+    if (z == 0) both(0);
+    else if (z == 1) both(1);
+    else if (z == 2) both(2);
+    else {
+      if (hp.dwf) {
+        R q5[12], w5[12], wq, ww;
+        hop5_load<P, DAG>(hp, v, i, s, rhs, q5, w5, wq, ww);
+        slot[3].put(q5, w5, wq, ww, x);
+      }
+      both(3);
+    }
+    if (z > 0) {
+      R a[12], b[12];
+      half_reals(gf, a);
+      half_reals(gb, b);
+      slot[z - 1].put(a, b, wf, wb, x);
+    }
+  }
+  __syncthreads();
+  if (z > 0) return;
+  R acc[24];
+  if (active) {
+    A acc_;
+    acc_.zero();
+    acc_.add(gf, 0, -sdag, wf);
+    acc_.add(gb, 0, sdag, wb);
+#pragma unroll
+    for (int mu = 1; mu < 4; mu++) {
+      R a[12], b[12];
+      slot[mu - 1].get(a, b, wf, wb, x);
+      reals_half(a, gf);
+      reals_half(b, gb);
+      acc_.add(gf, mu, -sdag, wf);
+      acc_.add(gb, mu, sdag, wb);
+    }
+    acc_.store(acc);
+    if (hp.dwf) {
+      R q5[12], w5[12], wq, ww;
+      slot[3].get(q5, w5, wq, ww, x);
+#pragma unroll
+      for (int k = 0; k < 12; k++) {
+        acc[k] += wq * q5[k];
+        acc[12 + k] += ww * w5[k];
+      }
+    }
+  }
+  constexpr int NV = ep_nred<EP>();
+  double red[NV > 0 ? NV : 1] = {};
+  hop_epilogue<P, EP, PR, PX>(hp, v, st, rhs, sl, s, i, active, acc, red);
+  if constexpr (NV > 0) {
+    // the block's values are this warp's
+    if (!ep_axpy(EP) || hp.norm) {
+      warp_sum(reinterpret_cast<double(&)[NV]>(red));
+      if (x == 0)
+#pragma unroll
+        for (int k = 0; k < NV; k++) partials[((size_t)rhs * nblk + sb) * NV + k] = red[k];
+    }
   }
 }
 

@@ -14,6 +14,7 @@ struct HopSel {
   bool dag;
   int ns;     // slices per thread (2: DWF slice pairs)
   bool halo;  // the t-slab decomposition's hop
+  bool split; // four threads per site (small lattices)
 };
 
 HopFn pick_hop_double(const HopSel &q);
@@ -22,6 +23,9 @@ HopFn pick_hop_half(const HopSel &q);
 
 template <int P, int RECON, int EP, int PR, int PX>
 HopFn get_hop(const HopSel &q) {
+  if constexpr (!ep_mix(EP)) {
+    if (q.split) return q.dag ? hop_split_kernel<P, RECON, EP, PR, PX, true> : hop_split_kernel<P, RECON, EP, PR, PX, false>;
+  }
   // FP32 arithmetic only: the FP64 pair kernel spills kilobytes
   if constexpr (!ep_mix(EP) && P != PREC_DOUBLE) {
     if (q.ns == 2)

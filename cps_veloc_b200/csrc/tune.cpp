@@ -11,6 +11,7 @@ struct Entry {
   TuneKey key;
   dim3 block;
   int order;
+  bool forced;  // set by the caller, not by the autotuner
 };
 std::vector<Entry> g_table;
 }  // namespace
@@ -41,15 +42,23 @@ int hop_order(const TuneKey &k) {
   return ORDER_SLICES;
 }
 
-void tune_set(const TuneKey &k, dim3 block, int order) {
+bool hop_forced(const TuneKey &k) {
+  std::lock_guard<std::mutex> lk(g_mu);
+  for (auto &e : g_table)
+    if (e.key == k) return e.forced;
+  return false;
+}
+
+void tune_set(const TuneKey &k, dim3 block, int order, bool forced) {
   std::lock_guard<std::mutex> lk(g_mu);
   for (auto &e : g_table)
     if (e.key == k) {
       e.block = block;
       e.order = order;
+      e.forced = forced;
       return;
     }
-  g_table.push_back({k, block, order});
+  g_table.push_back({k, block, order, forced});
 }
 
 void tune_clear() {

@@ -25,7 +25,10 @@ enum HopOrder { ORDER_SLICES = 0, ORDER_SITES = 1, ORDER_COUNT = 2 };
 
 dim3 hop_block(const TuneKey &k, bool mix);
 int hop_order(const TuneKey &k);
-void tune_set(const TuneKey &k, dim3 block, int order = ORDER_SLICES);
+// forced: the caller's own choice (cpsgpu_set_hop_shape); small launches keep
+// to it too, where a tuned or default shape gives way to hop_split_kernel
+void tune_set(const TuneKey &k, dim3 block, int order = ORDER_SLICES, bool forced = false);
+bool hop_forced(const TuneKey &k);
 void tune_clear();
 int tune_count();
 

@@ -621,7 +621,8 @@ int cpsgpu_set_rhs_tile(cpsgpu_dirac d, int prec, int tile);
  * CPSGPU_ORDER_SLICES (consecutive blocks: every slice group of one block
  * of sites) or CPSGPU_ORDER_SITES (consecutive blocks: the site blocks of
  * one slice group, lexicographically).  get returns the shape in use; set
- * overrides the autotuner.  The shape table (like the autotuner's) is shared by every
+ * overrides the autotuner (and the four-threads-per-site kernel that small
+ * launches of any other shape run).  The shape table (like the autotuner's) is shared by every
  * operator of the same kind, Ls, precision and link form. */
 enum { CPSGPU_ORDER_SLICES = 0, CPSGPU_ORDER_SITES = 1 };
 int cpsgpu_get_hop_shape(cpsgpu_dirac d, int prec, int *sites, int *slices, int *slices_per_thread, int *order);
