@@ -1,5 +1,7 @@
 #include "tune.h"
 
+#include "cpsgpu_impl.h"
+
 #include <mutex>
 #include <vector>
 
@@ -30,7 +32,16 @@ dim3 hop_block(const TuneKey &k, bool mix) {
     return dim3(p < 1 ? 1 : p, k.ls);
   }
   if (k.ls <= 1) return dim3(128, 1);
-  // 32 consecutive sites per warp; several slices per block share links in L1
+  // several slices of one 4D parity per block share their links in L1
+  if (k.kind == KIND_DWF) {
+    // 64 sites x 2 slices, FP64 32 x 4.  CG iteration with 64 x 2 / 32 x 4, two
+    // processes each: 16^3x32 Ls=16 FP32 498, 517 / 513, 525 us, FP16 437, 439
+    // / 439, 441, FP64 901, 956 / 944, 939; 12x14x20x22 Ls=12 FP32 244, 242 /
+    // 254, 248, FP16 213, 211 / 217, 215, FP64 427, 430 / 411, 411
+    if (k.ls % 4 == 0) return k.prec == PREC_DOUBLE ? dim3(32, 4) : dim3(64, 2);
+    // Ls = 6, 10, 14: an odd number of slices per parity, all of them
+    if (k.ls % 2 == 0 && k.ls <= 16) return dim3(32, k.ls / 2);
+  }
   int bs = (k.ls % 4 == 0) ? 4 : (k.ls % 2 == 0 ? 2 : 1);
   return dim3(32, bs);
 }
