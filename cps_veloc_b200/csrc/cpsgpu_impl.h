@@ -125,6 +125,16 @@ struct MobiusPlan {
   double coef = 0.0;
 };
 
+// A packed pair of real mixing matrices as out = a x + g y with y a shift of
+// x (BAND) or a recurrence along the slices (SCAN), per chirality (mix_scan.cu)
+struct MixScan {
+  enum { DENSE = 0, SCAN = 1, BAND = 2 };
+  int kind = DENSE;
+  double rho[2], w[2], a[2], g[2];
+  int down[2];  // 1: the recurrence starts at the last slice
+};
+MixScan fit_mix_scan(int ls, const std::vector<double> &packed);
+
 // Multishift CG workspace (multishift.cu), kept across calls on one operator.
 struct CgSolver;
 // an instantiated graph and the configuration it was captured for
@@ -193,6 +203,19 @@ struct Dirac {
   // host copy of every real mixing matrix uploaded for this operator, by
   // device address (launch_mix passes the matrix as a kernel parameter)
   std::unordered_map<const void *, std::vector<double>> mix_host;
+  // ... and its two-term form, where it has one
+  std::unordered_map<const void *, MixScan> mix_scan;
+  const MixScan *scan_of(const void *mix) const {
+    const auto it = mix_scan.find(mix);
+    return it == mix_scan.end() ? nullptr : &it->second;
+  }
+  // remember the host form of a real matrix just uploaded at ptr
+  void keep_mix(const void *ptr, const std::vector<double> &h) {
+    mix_host[ptr] = h;
+    const MixScan s = fit_mix_scan(ls, h);
+    if (s.kind != MixScan::DENSE) mix_scan[ptr] = s;
+    else mix_scan.erase(ptr);
+  }
   Dirac(Lattice *l, int kind_, int ls_, double mass_, double m5_, double b_, double c_, double a5inv_ = 1.0);
   // (re)build the Mobius matrices from per-slice coefficients
   void build_mobius(const std::vector<std::complex<double>> &bs, const std::vector<std::complex<double>> &cs);
@@ -259,6 +282,10 @@ MobiusTail mobius_head(const Dirac &D, int prec, int dag, const SpinorView &in, 
 bool mix_tc_applies(const Dirac &D, int prec);
 void launch_mix_tc(const Dirac &D, const double *mix, const SpinorView &in, const SpinorView &out,
                    const SolverScalars *st, int gate);
+// the recurrence along s of the matrices that have one (mix_scan.cu); false
+// when it does not apply
+bool launch_mix_scan(const Dirac &D, int prec, const double *mix, const SpinorView &in, const SpinorView &out,
+                     const SolverScalars *st, int gate);
 // out = Mix in (per chirality Ls x Ls), all slices
 // the register-tiled form of launch_mix (mix_reg.cu): real matrices whose
 // host copy is in D.mix_host and Ls among the instantiated sizes; false when

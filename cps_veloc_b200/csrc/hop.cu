@@ -51,6 +51,18 @@ void launch_hop(const Dirac &D, const HopLaunch &L, const SpinorView &in, const 
   for (int s = 0; s < D.ls && s < MAX_LS; s++) hp.coef[s] = L.coef.empty() ? 0.0 : L.coef[(size_t)s < L.coef.size() ? s : 0];
   hp.mix = L.mix;
   hp.mix_cplx = (L.mix != nullptr && D.cplx) ? 1 : 0;
+  const MixScan *scan = L.mix ? D.scan_of(L.mix) : nullptr;
+  if (scan) {
+    hp.scan = scan->kind;
+    for (int c = 0; c < 2; c++) {
+      const double v[4] = {scan->rho[c], scan->w[c], scan->a[c], scan->g[c]};
+      hp.scan_down[c] = scan->down[c];
+      for (int k = 0; k < 4; k++) {
+        hp.scan_d[c][k] = v[k];
+        hp.scan_f[c][k] = (float)v[k];
+      }
+    }
+  }
   hp.norm = L.norm;
   hp.red_op = L.red_op;
   hp.gate = L.gate;
@@ -113,7 +125,8 @@ void launch_hop(const Dirac &D, const HopLaunch &L, const SpinorView &in, const 
   dim3 grid = sites_first ? dim3(nsb * hp.rtile, hp.nsg, ntile) : dim3(nsb * hp.nsg * hp.rtile, 1, ntile);
   size_t smem = 0;
   if (mix) {
-    smem = (size_t)D.ls * block.x * 24 * real_size(L.prec) + 2 * (size_t)D.ls * D.ls * sizeof(double) * (D.cplx ? 2 : 1);
+    smem = (size_t)D.ls * block.x * 24 * real_size(L.prec);
+    if (!hp.scan) smem += 2 * (size_t)D.ls * D.ls * sizeof(double) * (D.cplx ? 2 : 1);
     // the attribute belongs to the kernel on one device: raised once per (device, kernel, size)
     struct Raised {
       int dev;

@@ -89,6 +89,12 @@ struct HopParams {
   double coef[MAX_LS];  // per-slice coefficient of the AXPY/CG/RES epilogues
   const double *mix;    // [2][ls][ls] row-major, upper then lower chirality ([..][re, im] if mix_cplx)
   int mix_cplx;         // complex mixing matrices (zMobius)
+  // the two-term form of the mixing (MixScan; mix_scan.cu), per chirality:
+  // rho, w, a, g in the arithmetic precisions
+  int scan;
+  int scan_down[2];
+  double scan_d[2][4];
+  float scan_f[2][4];
   int norm;         // AXPY: accumulate reductions
   int red_op;       // ReduceOp for the finalize
   int gate;         // Gate
@@ -470,6 +476,82 @@ __device__ __forceinline__ void hop_epilogue(const HopParams &hp, const HopViews
   }
 }
 
+// ---- the mixing epilogue's two-term form (MixScan, mix_scan.cu)
+template <typename R> struct Pair2;
+template <> struct Pair2<float> {
+  using T = float2;
+  static __device__ __forceinline__ T mk(float x, float y) { return make_float2(x, y); }
+  static __device__ __forceinline__ T fma(float s, T x, T y) { return __ffma2_rn(make_float2(s, s), x, y); }
+  static __device__ __forceinline__ T mul(float s, T x) { return __fmul2_rn(make_float2(s, s), x); }
+  static __device__ __forceinline__ const float *coef(const HopParams &hp, int c) { return hp.scan_f[c]; }
+};
+template <> struct Pair2<double> {
+  using T = double2;
+  static __device__ __forceinline__ T mk(double x, double y) { return make_double2(x, y); }
+  static __device__ __forceinline__ T fma(double s, T x, T y) { return make_double2(::fma(s, x.x, y.x), ::fma(s, x.y, y.y)); }
+  static __device__ __forceinline__ T mul(double s, T x) { return make_double2(s * x.x, s * x.y); }
+  static __device__ __forceinline__ const double *coef(const HopParams &hp, int c) { return hp.scan_d[c]; }
+};
+
+// acc <- Mix acc over the block's slices: staged as [ls][12][BX] pairs of
+// reals, one thread walks the slices of one (pair, site) column in place, and
+// every thread reads its slice back.  4 shared-memory words and 4 packed
+// multiply-adds per pair; the dense form takes Ls of each (Ls = 12: 144
+// 8-byte loads per thread against 36, stores included).  Called by every
+// thread of the block (s may be past the last slice).
+template <typename R>
+__device__ __forceinline__ void mix_scan_epilogue(const HopParams &hp, int s, bool active, R *acc, unsigned char *smraw) {
+  using Q = Pair2<R>;
+  using T = typename Q::T;
+  const int bx = blockDim.x, nthr = bx * blockDim.y, tid = threadIdx.x + bx * threadIdx.y, n = hp.ls;
+  T *sm = reinterpret_cast<T *>(smraw);
+  if (s < n) {
+    T *mine = sm + (size_t)s * 12 * bx + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < 12; k++) mine[k * bx] = active ? Q::mk(acc[2 * k], acc[2 * k + 1]) : Q::mk(R(0), R(0));
+  }
+  __syncthreads();
+  for (int q = tid; q < 12 * bx; q += nthr) {
+    const int c = q >= 6 * bx;
+    const R *cf = Q::coef(hp, c);
+    const R rho = cf[0], w = cf[1], a = cf[2], g = cf[3];
+    const int step = hp.scan_down[c] ? -12 * bx : 12 * bx;
+    T *col = sm + q + (hp.scan_down[c] ? (n - 1) * 12 * bx : 0);
+    const T x0 = col[0];
+    T x = x0, y;
+    if (hp.scan == 2) {  // MixScan::BAND
+      y = Q::mul(w, col[(n - 1) * step]);
+      for (int k = 0; k < n; k++) {
+        x = col[k * step];
+        col[k * step] = Q::fma(g, y, Q::mul(a, x));
+        y = x;
+      }
+    } else {
+      T h = x0;
+#pragma unroll 4
+      for (int k = 1; k < n; k++) h = Q::fma(rho, h, col[k * step]);
+      y = Q::fma(w, h, x0);
+      col[0] = Q::fma(g, y, Q::mul(a, x0));
+#pragma unroll 4
+      for (int k = 1; k < n; k++) {
+        x = col[k * step];
+        y = Q::fma(rho, y, x);
+        col[k * step] = Q::fma(g, y, Q::mul(a, x));
+      }
+    }
+  }
+  __syncthreads();
+  if (active) {
+    const T *mine = sm + (size_t)s * 12 * bx + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < 12; k++) {
+      const T v = mine[k * bx];
+      acc[2 * k] = v.x;
+      acc[2 * k + 1] = v.y;
+    }
+  }
+}
+
 // reductions of an epilogue: AXPY with norms 2, CG and RES 1, else none
 template <int EP> __host__ __device__ constexpr int ep_nred() {
   return ep_axpy(EP) ? 2 : (ep_cg(EP) || ep_res(EP)) ? 1 : 0;
@@ -573,6 +655,9 @@ __global__ void __launch_bounds__(256, (hop_min_blocks<P, NS>())) hop_kernel(con
   if constexpr (ep_mix(EP)) {
     // all Ls slices of this block's sites: out(s) = sum_t Mix_chi[s][t] acc(t)
     extern __shared__ unsigned char smraw[];
+    if (hp.scan) {
+      mix_scan_epilogue<R>(hp, s, active, acc, smraw);
+    } else {
     R *sm = reinterpret_cast<R *>(smraw);  // [ls][24][BX]: a warp's accesses are consecutive words
     double *mx = reinterpret_cast<double *>(sm + (size_t)hp.ls * blockDim.x * 24);
     const int tid = threadIdx.x + blockDim.x * threadIdx.y;
@@ -649,6 +734,7 @@ __global__ void __launch_bounds__(256, (hop_min_blocks<P, NS>())) hop_kernel(con
           }
         }
       }
+    }
     }
   }
 

@@ -261,9 +261,10 @@ void Dirac::build_mobius(const std::vector<cd> &bs, const std::vector<cd> &cs) {
   };
   // uploads keeping the host copy of a real matrix (launch_mix's parameter)
   mix_host.clear();
+  mix_scan.clear();
   auto upload = [&](DeviceBuffer &buf, const std::vector<double> &h) {
     cpsgpu::upload(buf, h);
-    if (!cplx) mix_host[buf.ptr] = h;
+    if (!cplx) keep_mix(buf.ptr, h);
   };
   hM5i = packm(m0u, m0d);
   hM5id = packm(m1u, m1d);
@@ -317,7 +318,10 @@ void Dirac::set_pc_type(int pc) {
   if (pc != PC_SYM2 && (cplx || !uniform_bc))
     throw Error(-1, "Mobius preconditioning other than SYM2: real b, c, the same on every slice");
   pc_type = pc;
-  for (const DeviceBuffer &b : pc_bufs) mix_host.erase(b.ptr);
+  for (const DeviceBuffer &b : pc_bufs) {
+    mix_host.erase(b.ptr);
+    mix_scan.erase(b.ptr);
+  }
   pc_bufs.clear();
   pc_bufs.reserve(16);
   plan[0] = plan[1] = MobiusPlan();
@@ -370,7 +374,7 @@ void Dirac::set_pc_type(int pc) {
     pc_bufs.emplace_back();
     const std::vector<double> h = pack(ls, a.u, a.d);
     upload(pc_bufs.back(), h);
-    mix_host[pc_bufs.back().ptr] = h;
+    keep_mix(pc_bufs.back().ptr, h);
     return pc_bufs.back().as<double>();
   };
   switch (pc) {

@@ -25,11 +25,21 @@ dim3 hop_block(const TuneKey &k, bool mix) {
       if (e.key == k) return e.block;
   }
   if (mix) {
-    // a block holds every slice of its sites
-    int bx = 256 / (k.ls > 0 ? k.ls : 1);
-    int p = 1;
-    while (p * 2 <= bx) p *= 2;
-    return dim3(p < 1 ? 1 : p, k.ls);
+    // a block holds every slice of its sites: a power of two of them, at most
+    // 192 threads (FP32) or 128 (FP64, FP16, while that leaves three warps):
+    // the barriers of the mixing stall one block at a time.  MatPcDagMatPc
+    // with 16 / 8 sites, Mobius 24^3x64 Ls=12: FP64 5.43 / 5.46 ms, FP32
+    // 2.35 / 2.45, FP16 1.84 / 1.79; 12^3x24 Ls=16: FP64 0.336 / 0.322, FP32
+    // 0.182 / 0.177; 10x6x14x18 Ls=10: FP32 62 / 64 us, FP16 63 / 68
+    const int ls = k.ls > 0 ? k.ls : 1;
+    auto pow2 = [&](int threads) {
+      int p = 1;
+      while (2 * p * ls <= threads) p *= 2;
+      return p;
+    };
+    int bx = pow2(k.prec == PREC_SINGLE ? 192 : 128);
+    if (bx * ls < 96) bx = pow2(192);
+    return dim3(bx, k.ls);
   }
   if (k.ls <= 1) return dim3(128, 1);
   // several slices of one 4D parity per block share their links in L1

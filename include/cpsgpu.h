@@ -245,6 +245,10 @@ int cpsgpu_dirac_get_pc_type(cpsgpu_dirac d, int *pc_type);
  *     the two real matrices are a kernel parameter, every thread computes
  *     all Ls output slices of a block of reals with packed FP32 multiply-adds
  *     (Ls 8, 10, 12, 16, 20, 24; real b, c); FP64 fields as 2.
+ * Matrices of one real b, c on every slice (|K| <= 1, Ls >= 3) run as a
+ * recurrence along the slices under 0, 2 and 3 alike (mix_scan.cu); the
+ * kernels named above then apply to the others (real b_s, c_s that differ
+ * between slices, and at FP16 the Ls that mix_scan.cu does not instantiate).
  * Every form but 1 gives the same bits. */
 int cpsgpu_set_mix_impl(cpsgpu_dirac d, int impl);
 
