@@ -10,6 +10,7 @@
 
 #include "../../include/cpsgpu.h"
 #include "cpsgpu_impl.h"
+#include "host_copy.h"
 #include "hop.cuh"
 #include "tune.h"
 #include "solver.h"
@@ -121,8 +122,7 @@ void upload(Lattice &L, Field &f, const double *const *host, int nrhs) {
   size_t n = (size_t)24 * f.vh * f.ls;
   L.staging.ensure(n * nrhs * sizeof(double));
   for (int k = 0; k < nrhs; k++)
-    CPSGPU_CUDA(cudaMemcpyAsync(L.staging.as<double>() + n * k, host[k], n * sizeof(double), cudaMemcpyHostToDevice,
-                                L.stream));
+    copy_to_device(L.stream, L.staging.as<double>() + n * k, host[k], n * sizeof(double));
   launch_import_fermion(L.stream, f.prec, f.view(), L.staging.as<double>());
 }
 
@@ -131,8 +131,7 @@ void download(Lattice &L, const Field &f, double *const *host, int nrhs) {
   L.staging.ensure(n * nrhs * sizeof(double));
   launch_export_fermion(L.stream, f.prec, f.view(), L.staging.as<double>());
   for (int k = 0; k < nrhs; k++)
-    CPSGPU_CUDA(cudaMemcpyAsync(host[k], L.staging.as<double>() + n * k, n * sizeof(double), cudaMemcpyDeviceToHost,
-                                L.stream));
+    copy_to_host(L.stream, host[k], L.staging.as<double>() + n * k, n * sizeof(double));
   CPSGPU_CUDA(cudaStreamSynchronize(L.stream));
 }
 
@@ -797,10 +796,10 @@ int cpsgpu_evolve_mom_fforce(cpsgpu_dirac d, double *mom, const double *chi, dou
     Lattice &L = *d->D->lat;
     const size_t bytes = (size_t)2 * L.vh * 4 * 18 * sizeof(double);
     d->mom.ensure(2 * bytes);
-    CPSGPU_CUDA(cudaMemcpyAsync(d->mom.ptr, mom, bytes, cudaMemcpyHostToDevice, L.stream));
+    copy_to_device(L.stream, d->mom.ptr, mom, bytes);
     double f[3];
     fforce_update(*d->D, fv, d->mom.as<double>(), dt, f);
-    CPSGPU_CUDA(cudaMemcpyAsync(mom, d->mom.ptr, bytes, cudaMemcpyDeviceToHost, L.stream));
+    copy_to_host(L.stream, mom, d->mom.ptr, bytes);
     CPSGPU_CUDA(cudaStreamSynchronize(L.stream));
     if (out) {
       out->L1 = f[0];
@@ -827,7 +826,7 @@ int cpsgpu_rhmc_evolve_mom_fforce(cpsgpu_dirac d, double *mom, const double *con
     const size_t bytes = (size_t)2 * L.vh * 4 * 18 * sizeof(double);
     d->mom.ensure(2 * bytes);
     double *m = d->mom.as<double>(), *tmp = m + bytes / sizeof(double);
-    CPSGPU_CUDA(cudaMemcpyAsync(m, mom, bytes, cudaMemcpyHostToDevice, L.stream));
+    copy_to_device(L.stream, m, mom, bytes);
     // FORCE_MEASURE_YES: the poles accumulate into a zeroed field whose norms
     // are measured before it is added to mom (f_wilson.C:689-757)
     double *acc = force_measure ? tmp : m;
@@ -841,7 +840,7 @@ int cpsgpu_rhmc_evolve_mom_fforce(cpsgpu_dirac d, double *mom, const double *con
       mom_norms(L, tmp, f);
       mom_add(L, m, tmp);
     }
-    CPSGPU_CUDA(cudaMemcpyAsync(mom, m, bytes, cudaMemcpyDeviceToHost, L.stream));
+    copy_to_host(L.stream, mom, m, bytes);
     CPSGPU_CUDA(cudaStreamSynchronize(L.stream));
     if (out) {
       out->L1 = f[0];

@@ -5,6 +5,7 @@
 #include <cstring>
 
 #include "cpsgpu_impl.h"
+#include "host_copy.h"
 #include "hop.cuh"
 
 namespace cpsgpu {
@@ -519,7 +520,7 @@ void import_gauge(Lattice &L, const double *host, int signs_applied) {
   L.gH12.ensure(nlinks * 12 * sizeof(__half));
   L.gS18.ensure(nlinks * 18 * sizeof(float));
   L.gH18.ensure(nlinks * 18 * sizeof(__half));
-  CPSGPU_CUDA(cudaMemcpyAsync(L.staging.ptr, host, nlinks * 18 * sizeof(double), cudaMemcpyHostToDevice, L.stream));
+  copy_to_device(L.stream, L.staging.ptr, host, nlinks * 18 * sizeof(double));
   DeviceBuffer err(sizeof(double));
   CPSGPU_CUDA(cudaMemsetAsync(err.ptr, 0, sizeof(double), L.stream));
   gauge_import_kernel<<<blocks_for(nlinks), TPB, 0, L.stream>>>(

@@ -22,6 +22,7 @@
 
 #include "../../include/cpsgpu.h"
 #include "cpsgpu_impl.h"
+#include "host_copy.h"
 #include "hop.cuh"
 #include "solver.h"
 
@@ -333,13 +334,13 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
   L.partials.ensure(nblk * 2 * sizeof(double));
 
   L.staging.ensure(nreal * sizeof(double));
-  CPSGPU_CUDA(cudaMemcpyAsync(L.staging.ptr, chi_h, nreal * sizeof(double), cudaMemcpyHostToDevice, s));
+  copy_to_device(s, L.staging.ptr, chi_h, nreal * sizeof(double));
   launch_import_fermion(s, PREC_DOUBLE, chi64.view(), L.staging.as<double>());
   Field psi0_64;  // GENERAL: the FP64 guess of shift 0 for the initial residual
   if (dev_type == 2) {
     // GENERAL accumulates into the given solutions (only MULTI zeroes them)
     for (int k = 0; k < npsi; k++) {
-      CPSGPU_CUDA(cudaMemcpyAsync(L.staging.ptr, psi_h[k], nreal * sizeof(double), cudaMemcpyHostToDevice, s));
+      copy_to_device(s, L.staging.ptr, psi_h[k], nreal * sizeof(double));
       if (PS == PREC_DOUBLE) {
         launch_import_fermion(s, PREC_DOUBLE, psi[k].view(), L.staging.as<double>());
       } else {
@@ -352,7 +353,7 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
   } else {
     for (int k = 0; k < npsi; k++) launch_zero(s, psi[k]);
     if (type == 0 && dev_type == 0) {
-      CPSGPU_CUDA(cudaMemcpyAsync(L.staging.ptr, psi_h[0], nreal * sizeof(double), cudaMemcpyHostToDevice, s));
+      copy_to_device(s, L.staging.ptr, psi_h[0], nreal * sizeof(double));
       launch_import_fermion(s, PREC_DOUBLE, psi[0].view(), L.staging.as<double>());
     }
   }
@@ -761,7 +762,7 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
     for (size_t q = 0; q < nreal; q++) acc[q] = psi_h[0][q];
     for (int k = 0; k < nshift; k++) {
       launch_export_fermion(s, PREC_DOUBLE, solution(k), L.staging.as<double>());
-      CPSGPU_CUDA(cudaMemcpyAsync(tmp.data(), L.staging.ptr, nreal * sizeof(double), cudaMemcpyDeviceToHost, s));
+      copy_to_host(s, tmp.data(), L.staging.ptr, nreal * sizeof(double));
       CPSGPU_CUDA(cudaStreamSynchronize(s));
       for (size_t q = 0; q < nreal; q++) acc[q] += alpha[k] * tmp[q];
     }
@@ -769,7 +770,7 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
   } else {
     for (int k = 0; k < npsi; k++) {
       launch_export_fermion(s, PREC_DOUBLE, solution(k), L.staging.as<double>());
-      CPSGPU_CUDA(cudaMemcpyAsync(psi_h[k], L.staging.ptr, nreal * sizeof(double), cudaMemcpyDeviceToHost, s));
+      copy_to_host(s, psi_h[k], L.staging.ptr, nreal * sizeof(double));
     }
     CPSGPU_CUDA(cudaStreamSynchronize(s));
   }
