@@ -251,6 +251,12 @@ template <> struct Slice<PREC_HALF> {
 #pragma unroll
     for (int g = 0; g < 3; g++) unpack8(__ldg(d + j + g * vh), s, v + 8 * g);
   }
+  // the three groups as stored, and the site's norm
+  __device__ __forceinline__ void load_groups(int j, uint4 (&q)[3], float &scale) const {
+    scale = __ldg(n + j);
+#pragma unroll
+    for (int g = 0; g < 3; g++) q[g] = __ldg(d + j + g * vh);
+  }
   // the stored values unscaled, and the site's norm: the caller folds the
   // norm into a multiply it does anyway (24 fewer multiplies per site)
   __device__ __forceinline__ void load_raw(int j, float *v, float &scale) const {
@@ -288,6 +294,21 @@ template <> struct Slice<PREC_HALF> {
       for (int k = 0; k < 12; k++) v[k] = tmp[4 + k];
     }
   }
+};
+
+// One site of a slice as the hop reads it: loaded first (its loads in flight
+// with the link's), projected when the link is there
+template <int P> struct Neighbour {
+  using R = typename PrecTraits<P>::real;
+  R psi[24], scale;
+  __device__ __forceinline__ Neighbour(const Slice<P> &in, int j) { in.load_raw(j, psi, scale); }
+  __device__ __forceinline__ half_spinor<R> proj(int mu, R k) const { return project(psi, mu, k); }
+};
+template <> struct Neighbour<PREC_HALF> {
+  uint4 q[3];
+  float scale;
+  __device__ __forceinline__ Neighbour(const Slice<PREC_HALF> &in, int j) { in.load_groups(j, q, scale); }
+  __device__ __forceinline__ half_spinor<float> proj(int mu, float k) const { return project_half(q, mu, k); }
 };
 
 // ---- 4-real chunks (reals 4c .. 4c+3) for register-light epilogues ----

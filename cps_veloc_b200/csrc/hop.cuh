@@ -203,12 +203,11 @@ __device__ __forceinline__ void hop_dir(const HopParams &hp, const HopViews &v, 
       g = A::mul(u, load_halo<R>(v.hf, hp.face, sl, j), false);
       w = (hp.tb_fwd && hp.bc[mu] < 0) ? R(-1) : R(1);
     } else {
-      R psi[24], sc;
-      in.load_raw(j, psi, sc);
+      const Neighbour<P> nb(in, j);
       su3<R> u;
       LinkIO<P, RECON>::load(v.U, pout, mu, i, u);
-      g = A::mul(u, project(psi, mu, -sdag), false);
-      w = (wrap && hp.bc[mu] < 0 && (!HALO || mu != 3 || hp.tb_fwd)) ? -sc : sc;
+      g = A::mul(u, nb.proj(mu, -sdag), false);
+      w = (wrap && hp.bc[mu] < 0 && (!HALO || mu != 3 || hp.tb_fwd)) ? -nb.scale : nb.scale;
     }
   } else {  // U_mu(x - mu)^dagger (1 + sdag g_mu) psi(x - mu)
     const bool wrap = (q.c[mu] == 0);
@@ -220,12 +219,11 @@ __device__ __forceinline__ void hop_dir(const HopParams &hp, const HopViews &v, 
       g = A::pack(load_halo<R>(v.hb, hp.face, sl, i));
       w = (hp.tb_bwd && hp.bc[mu] < 0) ? R(-1) : R(1);
     } else {
-      R psi[24], sc;
-      in.load_raw(j, psi, sc);
+      const Neighbour<P> nb(in, j);
       su3<R> u;
       LinkIO<P, RECON>::load(v.U, pin, mu, j, u);
-      g = A::mul(u, project(psi, mu, sdag), true);
-      w = (wrap && hp.bc[mu] < 0 && (!HALO || mu != 3 || hp.tb_bwd)) ? -sc : sc;
+      g = A::mul(u, nb.proj(mu, sdag), true);
+      w = (wrap && hp.bc[mu] < 0 && (!HALO || mu != 3 || hp.tb_bwd)) ? -nb.scale : nb.scale;
     }
   }
 }
@@ -284,13 +282,11 @@ __device__ __forceinline__ void hop_site2(const HopParams &hp, const HopViews &v
       if (mu == 0) j = i - xh + ((wrap ? 0 : x + 1) >> 1);
       else j = wrap ? i - (hp.L[mu] - 1) * stride[mu] : i + stride[mu];
       const R sgn = (wrap && hp.bc[mu] < 0) ? R(-1) : R(1);
-      R psi0[24], psi1[24], sc0, sc1;
-      in0.load_raw(j, psi0, sc0);
-      in1.load_raw(j, psi1, sc1);
+      const Neighbour<P> n0(in0, j), n1(in1, j);
       su3<R> u;
       LinkIO<P, RECON>::load(v.U, pout, mu, i, u);
-      A0.hop(u, project(psi0, mu, -sdag), false, mu, -sdag, sgn * sc0);
-      A1.hop(u, project(psi1, mu, -sdag), false, mu, -sdag, sgn * sc1);
+      A0.hop(u, n0.proj(mu, -sdag), false, mu, -sdag, sgn * n0.scale);
+      A1.hop(u, n1.proj(mu, -sdag), false, mu, -sdag, sgn * n1.scale);
     }
     {
       const bool wrap = (c[mu] == 0);
@@ -298,13 +294,11 @@ __device__ __forceinline__ void hop_site2(const HopParams &hp, const HopViews &v
       if (mu == 0) j = i - xh + ((wrap ? hp.L[0] - 1 : x - 1) >> 1);
       else j = wrap ? i + (hp.L[mu] - 1) * stride[mu] : i - stride[mu];
       const R sgn = (wrap && hp.bc[mu] < 0) ? R(-1) : R(1);
-      R psi0[24], psi1[24], sc0, sc1;
-      in0.load_raw(j, psi0, sc0);
-      in1.load_raw(j, psi1, sc1);
+      const Neighbour<P> n0(in0, j), n1(in1, j);
       su3<R> u;
       LinkIO<P, RECON>::load(v.U, pin, mu, j, u);
-      A0.hop(u, project(psi0, mu, sdag), true, mu, sdag, sgn * sc0);
-      A1.hop(u, project(psi1, mu, sdag), true, mu, sdag, sgn * sc1);
+      A0.hop(u, n0.proj(mu, sdag), true, mu, sdag, sgn * n0.scale);
+      A1.hop(u, n1.proj(mu, sdag), true, mu, sdag, sgn * n1.scale);
     }
   }
   A0.store(acc0);
