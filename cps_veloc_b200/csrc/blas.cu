@@ -82,10 +82,10 @@ __global__ void zero_kernel(SpinorView dst, size_t n) {
 // row; with the finalize's narrower blocks CG on Wilson 8^3x16 went from 41.7
 // to 38.0 us per iteration in FP64, 42.0 to 38.2 with the FP32 inner solve)
 template <int P>
-__global__ void __launch_bounds__(TPB) xpay_kernel(SpinorView p, SpinorView r, const SolverScalars *st, size_t per) {
+__global__ void __launch_bounds__(TPB) xpay_kernel(SpinorView p, SpinorView r, const SolverScalars *st, size_t per, int rev) {
   using R = RealT<P>;
   constexpr int N = 16 / sizeof(R);
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t idx = (size_t)(rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * blockDim.x + threadIdx.x;
   const int rhs = (int)(blockIdx.y);
   if (st[rhs].done) return;
   if (idx >= per) return;
@@ -103,8 +103,8 @@ __global__ void __launch_bounds__(TPB) xpay_kernel(SpinorView p, SpinorView r, c
 // FP16 (a norm per site): a thread per site
 template <>
 __global__ void __launch_bounds__(TPB) xpay_kernel<PREC_HALF>(SpinorView p, SpinorView r, const SolverScalars *st,
-                                                             size_t per) {
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+                                                             size_t per, int rev) {
+  const size_t idx = (size_t)(rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * blockDim.x + threadIdx.x;
   const int rhs = (int)(blockIdx.y);
   if (st[rhs].done) return;
   if (idx >= per) return;
@@ -409,13 +409,13 @@ void launch_zero(cudaStream_t s, const Field &f) {
   launch_counter()++;
 }
 
-void launch_xpay(cudaStream_t s, int prec, const SpinorView &p, const SpinorView &r, SolverScalars *st, int nrhs) {
+void launch_xpay(cudaStream_t s, int prec, const SpinorView &p, const SpinorView &r, SolverScalars *st, int nrhs, int rev) {
   const size_t sites = (size_t)p.vh * p.ls;
   const size_t per = prec == PREC_DOUBLE ? 12 * sites : prec == PREC_SINGLE ? 6 * sites : sites;
   dim3 grid(blocks_for(per), nrhs);
-  if (prec == PREC_DOUBLE) xpay_kernel<PREC_DOUBLE><<<grid, TPB, 0, s>>>(p, r, st, per);
-  else if (prec == PREC_SINGLE) xpay_kernel<PREC_SINGLE><<<grid, TPB, 0, s>>>(p, r, st, per);
-  else xpay_kernel<PREC_HALF><<<grid, TPB, 0, s>>>(p, r, st, per);
+  if (prec == PREC_DOUBLE) xpay_kernel<PREC_DOUBLE><<<grid, TPB, 0, s>>>(p, r, st, per, rev);
+  else if (prec == PREC_SINGLE) xpay_kernel<PREC_SINGLE><<<grid, TPB, 0, s>>>(p, r, st, per, rev);
+  else xpay_kernel<PREC_HALF><<<grid, TPB, 0, s>>>(p, r, st, per, rev);
   CPSGPU_CUDA(cudaGetLastError());
   launch_counter()++;
 }

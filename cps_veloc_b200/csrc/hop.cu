@@ -63,6 +63,7 @@ void launch_hop(const Dirac &D, const HopLaunch &L, const SpinorView &in, const 
       }
     }
   }
+  hp.rev = lat.turn();
   hp.norm = L.norm;
   hp.red_op = L.red_op;
   hp.gate = L.gate;

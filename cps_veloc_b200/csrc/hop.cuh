@@ -111,6 +111,7 @@ struct HopParams {
   // slab (their hops need no halo); SUB_BOUNDARY its first and last
   // t-slices, subn site blocks each
   int sub, subn;
+  int rev;          // 1: the blocks take the sites from the last to the first (Lattice::turn)
   int i0, iend, jump;  // first site, end of the (first) site range, the boundary subset's jump
 };
 
@@ -583,17 +584,19 @@ __global__ void __launch_bounds__(256, (hop_min_blocks<P, NS>())) hop_kernel(con
   // tile), rhs fastest; ORDER_SITES: blockIdx.x = (site block, rhs),
   // blockIdx.y = slice group.  Either way consecutive blocks read the same
   // links (rtile solves) and sb numbers the blocks of one solve.
-  const int rin = blockIdx.x % hp.rtile, sbx = blockIdx.x / hp.rtile;
+  const int rin = blockIdx.x % hp.rtile;
+  const unsigned nbx = gridDim.x / hp.rtile;
+  const int sbx = hp.rev ? (int)(nbx - 1 - blockIdx.x / hp.rtile) : (int)(blockIdx.x / hp.rtile);
+  const int by = hp.rev ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y;
   const long rhs = (long)blockIdx.z * hp.rtile + rin;
   if (rhs >= hp.nrhs) return;  // the last tile may be partial
   if (hp.gate == GATE_RUNNING && st[rhs].done) return;
   if (hp.gate == GATE_RELIABLE && (st[rhs].done || !st[rhs].reliable)) return;
-  const unsigned nbx = gridDim.x / hp.rtile;
   const unsigned nblk = nbx * gridDim.y;  // blocks of one solve
-  const int sb = (int)(blockIdx.y * nbx) + sbx;
+  const int sb = by * (int)nbx + sbx;
   int sgrp, sblk;
   if (gridDim.y > 1) {
-    sgrp = blockIdx.y;
+    sgrp = by;
     sblk = sbx;
   } else {
     sgrp = sbx % hp.nsg;

@@ -58,7 +58,7 @@ constexpr int SCAN_SITES = 32;
 template <int P, int LS, bool BAND>
 __global__ void __launch_bounds__(SCAN_SITES * PrecTraits<P>::NG)
     scan_kernel(SpinorView in, SpinorView out, const ScanArg<typename PrecTraits<P>::real> arg, int ls,
-                const SolverScalars *st, int gate) {
+                const SolverScalars *st, int gate, int rev) {
   using R = typename PrecTraits<P>::real;
   using T = typename std::conditional<P == PREC_DOUBLE, double2, float4>::type;
   constexpr int NG = PrecTraits<P>::NG;
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(SCAN_SITES * PrecTraits<P>::NG)
   if (gate == GATE_RELIABLE && (st[blockIdx.z].done || !st[blockIdx.z].reliable)) return;
   const int n = LS > 0 ? LS : ls;
   const int g = threadIdx.y;
-  const long i = (long)blockIdx.x * SCAN_SITES + threadIdx.x;
+  const long i = (long)(rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * SCAN_SITES + threadIdx.x;
   if (i >= in.vh) return;
   const ScanCoef<R> c = arg.c[g >= NG / 2];  // uniform in a warp
   const long rhs = blockIdx.z, step = (c.down ? -1L : 1L) * NG * in.vh;
@@ -130,11 +130,11 @@ __device__ __forceinline__ void unpack12(const Half12 &v, int lower, float2 (&f)
 
 template <int LS, bool BAND>
 __global__ void __launch_bounds__(SCAN_HALF_TPB)
-    scan_half_kernel(SpinorView in, SpinorView out, const ScanArg<float> arg, const SolverScalars *st, int gate) {
+    scan_half_kernel(SpinorView in, SpinorView out, const ScanArg<float> arg, const SolverScalars *st, int gate, int rev) {
   if (gate == GATE_RUNNING && st[blockIdx.z].done) return;
   if (gate == GATE_RELIABLE && (st[blockIdx.z].done || !st[blockIdx.z].reliable)) return;
   const int lane = threadIdx.x & 31, lower = lane >> 4;
-  const int i = blockIdx.x * (SCAN_HALF_TPB / 2) + (threadIdx.x >> 5) * 16 + (lane & 15);
+  const int i = (rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * (SCAN_HALF_TPB / 2) + (threadIdx.x >> 5) * 16 + (lane & 15);
   const int vh = (int)in.vh;
   const bool active = i < vh;
   const ScanCoef<float> c = arg.c[lower];
@@ -253,22 +253,22 @@ template <typename R> ScanArg<R> scan_arg(const MixScan &m) {
 
 template <int P, int LS>
 void launch_full(const MixScan &m, const SpinorView &in, const SpinorView &out, int ls, const SolverScalars *st, int gate,
-                 cudaStream_t s) {
+                 cudaStream_t s, int rev) {
   using R = typename PrecTraits<P>::real;
   const ScanArg<R> a = scan_arg<R>(m);
   const dim3 block(SCAN_SITES, PrecTraits<P>::NG);
   const dim3 grid((unsigned)((in.vh + SCAN_SITES - 1) / SCAN_SITES), 1, in.nrhs);
-  if (m.kind == MixScan::BAND) scan_kernel<P, LS, true><<<grid, block, 0, s>>>(in, out, a, ls, st, gate);
-  else scan_kernel<P, LS, false><<<grid, block, 0, s>>>(in, out, a, ls, st, gate);
+  if (m.kind == MixScan::BAND) scan_kernel<P, LS, true><<<grid, block, 0, s>>>(in, out, a, ls, st, gate, rev);
+  else scan_kernel<P, LS, false><<<grid, block, 0, s>>>(in, out, a, ls, st, gate, rev);
 }
 
 template <int LS>
 void launch_half(const MixScan &m, const SpinorView &in, const SpinorView &out, const SolverScalars *st, int gate,
-                 cudaStream_t s) {
+                 cudaStream_t s, int rev) {
   const ScanArg<float> a = scan_arg<float>(m);
   const dim3 grid((unsigned)((in.vh + SCAN_HALF_TPB / 2 - 1) / (SCAN_HALF_TPB / 2)), 1, in.nrhs);
-  if (m.kind == MixScan::BAND) scan_half_kernel<LS, true><<<grid, SCAN_HALF_TPB, 0, s>>>(in, out, a, st, gate);
-  else scan_half_kernel<LS, false><<<grid, SCAN_HALF_TPB, 0, s>>>(in, out, a, st, gate);
+  if (m.kind == MixScan::BAND) scan_half_kernel<LS, true><<<grid, SCAN_HALF_TPB, 0, s>>>(in, out, a, st, gate, rev);
+  else scan_half_kernel<LS, false><<<grid, SCAN_HALF_TPB, 0, s>>>(in, out, a, st, gate, rev);
 }
 
 // one chirality; m(i, j) the matrix seen from the end the recurrence starts at
@@ -338,15 +338,16 @@ bool launch_mix_scan(const Dirac &D, int prec, const double *mix, const SpinorVi
   const MixScan *m = D.scan_of(mix);
   if (!m || in.ls != D.ls) return false;
   const cudaStream_t s = D.lat->stream;
+  const int rev = D.lat->turn();
   // the usual fifth extents in registers; others read the input twice (FP64,
   // FP32), or take the dense kernels (FP16)
   switch (D.ls) {
   // (FP16 keeps LS / 2 outputs too: up to Ls = 16 without spills)
 #define CPSGPU_SCAN_LS(N)                                                                     \
   case N:                                                                                     \
-    if (prec == PREC_DOUBLE) launch_full<PREC_DOUBLE, N>(*m, in, out, N, st, gate, s);        \
-    else if (prec == PREC_SINGLE) launch_full<PREC_SINGLE, N>(*m, in, out, N, st, gate, s);   \
-    else if constexpr (N <= 16) launch_half<N>(*m, in, out, st, gate, s);                     \
+    if (prec == PREC_DOUBLE) launch_full<PREC_DOUBLE, N>(*m, in, out, N, st, gate, s, rev);        \
+    else if (prec == PREC_SINGLE) launch_full<PREC_SINGLE, N>(*m, in, out, N, st, gate, s, rev);   \
+    else if constexpr (N <= 16) launch_half<N>(*m, in, out, st, gate, s, rev);                     \
     else return false;                                                                        \
     break;
     CPSGPU_SCAN_LS(4)
@@ -361,8 +362,8 @@ bool launch_mix_scan(const Dirac &D, int prec, const double *mix, const SpinorVi
     CPSGPU_SCAN_LS(24)
 #undef CPSGPU_SCAN_LS
     default:
-      if (prec == PREC_DOUBLE) launch_full<PREC_DOUBLE, 0>(*m, in, out, D.ls, st, gate, s);
-      else if (prec == PREC_SINGLE) launch_full<PREC_SINGLE, 0>(*m, in, out, D.ls, st, gate, s);
+      if (prec == PREC_DOUBLE) launch_full<PREC_DOUBLE, 0>(*m, in, out, D.ls, st, gate, s, rev);
+      else if (prec == PREC_SINGLE) launch_full<PREC_SINGLE, 0>(*m, in, out, D.ls, st, gate, s, rev);
       else return false;
   }
   CPSGPU_CUDA(cudaGetLastError());

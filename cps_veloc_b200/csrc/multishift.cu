@@ -155,10 +155,10 @@ struct MsRing {
 // psi_0 += f p_0, p_0 = r + a p_0; nothing when that iteration did not run
 template <int P>
 __global__ void __launch_bounds__(256) ms_lead_kernel(const void *r, void *p0, void *psi0, const MsScalars *ms, int slot,
-                                                       size_t n) {
+                                                       size_t n, int rev) {
   using V = MsVec<P>;
   if (ms->nh != slot + 1) return;
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t idx = (size_t)(rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= n) return;
   const bool upd = ms->h_upd[slot][0], adv = ms->h_adv[slot][0];
   typename V::T *pp = reinterpret_cast<typename V::T *>(p0) + idx, *yp = reinterpret_cast<typename V::T *>(psi0) + idx;
@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(256) ms_lead_kernel(const void *r, void *p0, v
 // arithmetic.  SUM: one solution, psi_0 += sum_s f_s p_s (type SINGLE).
 template <int P, bool SUM>
 __global__ void __launch_bounds__(256) ms_flush_kernel(const MsRing ring, const SpinorView *pv, const SpinorView *psiv,
-                                                       const MsScalars *ms, size_t n) {
+                                                       const MsScalars *ms, size_t n, int rev) {
   using V = MsVec<P>;
   using T = typename V::T;
   using R = RealT<P>;
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(256) ms_flush_kernel(const MsRing ring, const 
     a[j][s] = R(ms->ha[j][s]);
   }
   __syncthreads();
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t idx = (size_t)(rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= n) return;
   R r[MS_DEFER][V::N];
 #pragma unroll
@@ -503,8 +503,8 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
       const SpinorView rnew = slot_r(slot);
       launch_hop(D, Lh, hop_in, rnew, x, slot_r((slot + MS_DEFER - 1) % MS_DEFER), SpinorView(), in, SpinorView(), st);
       const unsigned g = (unsigned)((nvec + 255) / 256);
-      if (P == PREC_DOUBLE) ms_lead_kernel<PREC_DOUBLE><<<g, 256, 0, s>>>(rnew.data, p[0].data.ptr, psi[0].data.ptr, msd, slot, nvec);
-      else ms_lead_kernel<PREC_SINGLE><<<g, 256, 0, s>>>(rnew.data, p[0].data.ptr, psi[0].data.ptr, msd, slot, nvec);
+      auto lead = P == PREC_DOUBLE ? ms_lead_kernel<PREC_DOUBLE> : ms_lead_kernel<PREC_SINGLE>;
+      lead<<<g, 256, 0, s>>>(rnew.data, p[0].data.ptr, psi[0].data.ptr, msd, slot, nvec, L.turn());
       CPSGPU_CUDA(cudaGetLastError());
       launch_counter()++;
       return;
@@ -533,13 +533,10 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
     MsRing ring;
     for (int j = 0; j < MS_DEFER; j++) ring.r[j] = slot_r(j).data;
     const unsigned g = (unsigned)((nvec + 255) / 256);
-    if (dev_type == 0) {
-      ms_flush_kernel<PREC_DOUBLE, true><<<g, 256, 0, s>>>(ring, pvd.as<SpinorView>(), psivd.as<SpinorView>(), msd, nvec);
-    } else if (P == PREC_DOUBLE) {
-      ms_flush_kernel<PREC_DOUBLE, false><<<g, 256, 0, s>>>(ring, pvd.as<SpinorView>(), psivd.as<SpinorView>(), msd, nvec);
-    } else {
-      ms_flush_kernel<PREC_SINGLE, false><<<g, 256, 0, s>>>(ring, pvd.as<SpinorView>(), psivd.as<SpinorView>(), msd, nvec);
-    }
+    auto kernel = dev_type == 0       ? ms_flush_kernel<PREC_DOUBLE, true>
+                  : P == PREC_DOUBLE ? ms_flush_kernel<PREC_DOUBLE, false>
+                                     : ms_flush_kernel<PREC_SINGLE, false>;
+    kernel<<<g, 256, 0, s>>>(ring, pvd.as<SpinorView>(), psivd.as<SpinorView>(), msd, nvec, L.turn());
     CPSGPU_CUDA(cudaGetLastError());
     launch_counter()++;
   };

@@ -245,7 +245,7 @@ void CgSolver::emit_iteration(bool conditional) {
       launch_counter() = b0;  // counted when a body runs
     }
   }
-  launch_xpay(L.stream, sloppy, p.view(), r.view(), stp, nrhs);
+  launch_xpay(L.stream, sloppy, p.view(), r.view(), stp, nrhs, L.turn());
 }
 
 // Poll the done flags of all right-hand sides (pinned copy issued earlier).
