@@ -12,12 +12,14 @@
 // MatPcDagMatPc, DWF 8^4 Ls=8 (6 MB) 0.46 / 0.28 ms; 12 batched solves on
 // 8^3x16 (226 MB) 48.3 / 38.2 ms
 //
-// The ring (RING chunks of at most CHUNK bytes, 32 MiB) and the threads
+// The ring (RING chunks of at most CHUNK bytes, 16 MiB) and the threads
 // belong to one device; they are made by the first copy that needs them,
 // shared by every lattice of the device and given back when the last lattice
 // goes.  One transfer uses them at a time: a second thread's transfer that
 // finds them busy takes the driver's path.
 #include "host_copy.h"
+
+#include <sched.h>
 
 #include <atomic>
 #include <condition_variable>
@@ -35,7 +37,10 @@ namespace cpsgpu {
 
 namespace {
 
-constexpr size_t CHUNK = size_t(4) << 20;
+constexpr size_t CHUNK = size_t(2) << 20;
+// 8 x 4 MiB copies no faster and its pinning showed: making an 8^4 lattice and
+// uploading to it 31 ms, with 8 x 2 MiB 15; the force with 8 x 1 MiB 8.8 ms, with
+// 5 x 2 MiB 8.0, with 8 x 2 MiB 7.3
 constexpr int RING = 8;
 // below this the driver's path is as fast (one chunk, no overlap)
 constexpr size_t SMALLEST = size_t(256) << 10;
@@ -108,6 +113,14 @@ class CopyPool {
   size_t n_ = 0;
 };
 
+// the cores this process may run on (its affinity mask, which containers set)
+int usable_cores() {
+  cpu_set_t set;
+  CPU_ZERO(&set);
+  if (sched_getaffinity(0, sizeof(set), &set) == 0) return CPU_COUNT(&set);
+  return (int)std::thread::hardware_concurrency();
+}
+
 struct Stager {
   std::mutex busy;
   char *ring = nullptr;
@@ -123,9 +136,9 @@ struct Stager {
   // the buffers and threads; false when the host has none to give
   bool ready() {
     if (ring) return true;
-    const unsigned hc = std::thread::hardware_concurrency();
+    const int cores = usable_cores();
     try {
-      if (!pool) pool.reset(new CopyPool(hc >= 16 ? 7 : hc >= 4 ? (int)hc / 2 - 1 : 0));
+      if (!pool) pool.reset(new CopyPool(cores >= 16 ? 7 : cores >= 4 ? cores / 2 - 1 : 0));
     } catch (const std::exception &) {
       return false;  // no threads: the driver's path
     }
