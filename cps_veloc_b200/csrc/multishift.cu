@@ -435,8 +435,14 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
       size_t free_b = 0, total_b = 0;
       CPSGPU_CUDA(cudaMemGetInfo(&free_b, &total_b));
       if ((MS_DEFER - 1) * one_field > free_b / 4) return;
-      mw.ring.resize(MS_DEFER - 1);
-      for (auto &f : mw.ring) f.create(P, vh, ls, 1);
+      try {
+        mw.ring.resize(MS_DEFER - 1);
+        for (auto &f : mw.ring) f.create(P, vh, ls, 1);
+      } catch (const Error &) {  // another allocation was first: no ring
+        cudaGetLastError();
+        mw.ring.clear();
+        return;
+      }
     }
     deferred = true;
   };
