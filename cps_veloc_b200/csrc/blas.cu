@@ -41,9 +41,10 @@ long long &launch_counter() {
   return n;
 }
 
-void ensure_field(Field &f, int prec, long vh, int ls, int nrhs) {
-  if (f.data.ptr && f.prec == prec && f.vh == vh && f.ls == ls && f.nrhs == nrhs) return;
+bool ensure_field(Field &f, int prec, long vh, int ls, int nrhs) {
+  if (f.data.ptr && f.prec == prec && f.vh == vh && f.ls == ls && f.nrhs == nrhs) return false;
   f.create(prec, vh, ls, nrhs);
+  return true;
 }
 
 namespace {

@@ -45,7 +45,12 @@ struct DeviceBuffer {
     if (n) CPSGPU_CUDA(cudaMalloc(&ptr, n));
     bytes = n;
   }
-  void ensure(size_t n) { if (n > bytes) alloc(n); }
+  // at least n bytes; true when the buffer was made anew
+  bool ensure(size_t n) {
+    if (n <= bytes) return false;
+    alloc(n);
+    return true;
+  }
   void release() { if (ptr) cudaFree(ptr); ptr = nullptr; bytes = 0; }
   template <typename T> T *as() const { return reinterpret_cast<T *>(ptr); }
 };
@@ -174,8 +179,10 @@ struct MsWork {
   Field chi, r, tmp;
   std::vector<Field> p, psi;
   std::vector<Field> ring;  // residuals of a chunk's iterations (deferred updates); the last is r
-  DeviceBuffer st, ms, pv, psiv;
+  DeviceBuffer st, ms, pv, psiv, partials;
   OpWork w;
+  // The graphs hold the addresses of the buffers above: whichever of those is
+  // made anew drops both (minvcg), so neither key needs an address.
   // the recurrences' loop: a WHILE node over chunks of iterations, ctl its
   // [bodies run, bound] counters
   CachedGraph loop;
@@ -411,6 +418,6 @@ void mom_add(Lattice &L, double *mom, const double *x);
 long long &launch_counter();
 
 // workspace sizing helper
-void ensure_field(Field &f, int prec, long vh, int ls, int nrhs);
+bool ensure_field(Field &f, int prec, long vh, int ls, int nrhs);
 
 }  // namespace cpsgpu

@@ -315,23 +315,35 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
 
   // workspace kept on the operator across calls (allocated on first use)
   MsWork &mw = D.ms;
+  auto drop_graphs = [&] {
+    mw.loop.drop();
+    mw.full.drop();
+  };
+  auto field = [&](Field &f, int prec) {
+    if (ensure_field(f, prec, vh, ls, 1)) drop_graphs();
+  };
+  auto buffer = [&](DeviceBuffer &b, size_t bytes) {
+    if (b.ensure(bytes)) drop_graphs();
+  };
   Field &chi64 = mw.chi, &r = mw.r, &tmp64 = mw.tmp;
-  ensure_field(chi64, PREC_DOUBLE, vh, ls, 1);
-  ensure_field(r, P, vh, ls, 1);
-  ensure_field(tmp64, PREC_DOUBLE, vh, ls, 1);
+  field(chi64, PREC_DOUBLE);
+  field(r, P);
+  field(tmp64, PREC_DOUBLE);
   if (mw.p.size() < (size_t)nshift) mw.p.resize(nshift);
   if (mw.psi.size() < (size_t)npsi) mw.psi.resize(npsi);
   std::vector<Field> &p = mw.p, &psi = mw.psi;
-  for (int k = 0; k < nshift; k++) ensure_field(p[k], P, vh, ls, 1);
+  for (int k = 0; k < nshift; k++) field(p[k], P);
   const int PS = P;  // precision of the solutions during the recurrences
-  for (int k = 0; k < npsi; k++) ensure_field(psi[k], PS, vh, ls, 1);
+  for (int k = 0; k < npsi; k++) field(psi[k], PS);
   OpWork &w = mw.w;
-  ensure_field(w.t1, P, vh, ls, 1);
-  ensure_field(w.t2, P, vh, ls, 1);
-  if (D.kind == KIND_MOBIUS) ensure_field(w.t0, P, vh, ls, 1);
-  if (D.kind == KIND_MOBIUS && (D.plan[0].xmix || D.plan[1].xmix)) ensure_field(w.t3, P, vh, ls, 1);
-  size_t nblk = (size_t)((vh + 31) / 32) * ls + 1024;
-  L.partials.ensure(nblk * 2 * sizeof(double));
+  field(w.t1, P);
+  field(w.t2, P);
+  if (D.kind == KIND_MOBIUS) field(w.t0, P);
+  if (D.kind == KIND_MOBIUS && (D.plan[0].xmix || D.plan[1].xmix)) field(w.t3, P);
+  // the operator's own, as the graphs hold its address: the lattice's buffer
+  // moves when a larger solve on the lattice makes it grow
+  const size_t nblk = (size_t)((vh + 31) / 32) * ls + 1024;
+  buffer(mw.partials, nblk * 2 * sizeof(double));
 
   L.staging.ensure(nreal * sizeof(double));
   copy_to_device(s, L.staging.ptr, chi_h, nreal * sizeof(double));
@@ -358,8 +370,8 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
     }
   }
 
-  mw.st.ensure(sizeof(SolverScalars));
-  mw.ms.ensure(sizeof(MsScalars));
+  buffer(mw.st, sizeof(SolverScalars));
+  buffer(mw.ms, sizeof(MsScalars));
   SolverScalars *st = mw.st.as<SolverScalars>();
   MsScalars *msd = mw.ms.as<MsScalars>();
   SolverScalars st0;
@@ -410,8 +422,8 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
   std::vector<SpinorView> pv(nshift), psiv(npsi);
   for (int k = 0; k < nshift; k++) pv[k] = p[k].view();
   for (int k = 0; k < npsi; k++) psiv[k] = psi[k].view();
-  mw.pv.ensure(sizeof(SpinorView) * MS_MAX);
-  mw.psiv.ensure(sizeof(SpinorView) * MS_MAX);
+  buffer(mw.pv, sizeof(SpinorView) * MS_MAX);
+  buffer(mw.psiv, sizeof(SpinorView) * MS_MAX);
   DeviceBuffer &pvd = mw.pv, &psivd = mw.psiv;
   CPSGPU_CUDA(cudaMemcpyAsync(pvd.ptr, pv.data(), sizeof(SpinorView) * nshift, cudaMemcpyHostToDevice, s));
   CPSGPU_CUDA(cudaMemcpyAsync(psivd.ptr, psiv.data(), sizeof(SpinorView) * npsi, cudaMemcpyHostToDevice, s));
@@ -431,6 +443,7 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
     const bool have = mw.ring.size() == MS_DEFER - 1 && mw.ring[0].data.ptr && mw.ring[0].prec == P &&
                       mw.ring[0].vh == vh && mw.ring[0].ls == ls;
     if (!have) {
+      drop_graphs();
       mw.ring.clear();
       size_t free_b = 0, total_b = 0;
       CPSGPU_CUDA(cudaMemGetInfo(&free_b, &total_b));
@@ -459,6 +472,7 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
     HopLaunch Lh;
     Lh.prec = P;
     Lh.gate = GATE_RUNNING;
+    Lh.partials = mw.partials.as<double>();
     Lh.dag = 0;
     const SpinorView in = p[0].view();
     SpinorView hop_in = w.t1.view(), x = in;
@@ -550,13 +564,10 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
   CPSGPU_CUDA(cudaStreamSynchronize(s));
   const clk::time_point t_rec = clk::now();
   constexpr int chunk = MS_DEFER;
-  mw.ctl.ensure(2 * sizeof(int));
+  buffer(mw.ctl, 2 * sizeof(int));
   const int hctl[2] = {0, (int)std::min<long>((long)max_num_iter / chunk + 4, 1L << 30)};
   auto graph_key = [&]() -> std::vector<long long> {
-    return {P, nshift, dev_type, L.recon(P), D.pc_type, D.cplx ? 1 : 0,
-            (long long)(size_t)r.data.ptr, (long long)(size_t)w.t1.data.ptr,
-            (long long)(size_t)p[0].data.ptr, (long long)(size_t)psi[0].data.ptr,
-            deferred ? (long long)(size_t)mw.ring[0].data.ptr : 0};
+    return {P, nshift, dev_type, L.recon(P), D.pc_type, D.cplx ? 1 : 0, deferred ? 1 : 0};
   };
   // the recurrences as a WHILE node of graph g (after deps): chunks of
   // iterations until the solve is done, no host polling; returns the node
