@@ -21,16 +21,12 @@
 
 #include <sched.h>
 
-#include <atomic>
-#include <condition_variable>
-#include <cstdint>
-#include <cstring>
 #include <map>
 #include <memory>
 #include <mutex>
 #include <thread>
-#include <vector>
 
+#include "copy_pool.h"
 #include "cpsgpu_impl.h"
 
 namespace cpsgpu {
@@ -45,74 +41,6 @@ constexpr int RING = 8;
 // below this the driver's path is as fast (one chunk, no overlap)
 constexpr size_t SMALLEST = size_t(256) << 10;
 
-// memcpy split over the calling thread and a few workers
-class CopyPool {
- public:
-  explicit CopyPool(int workers) {
-    for (int k = 0; k < workers; k++) th_.emplace_back([this, k] { work(k); });
-  }
-  ~CopyPool() {
-    {
-      std::lock_guard<std::mutex> lk(mu_);
-      quit_ = true;
-      gen_.fetch_add(1, std::memory_order_release);
-    }
-    cv_.notify_all();
-    for (auto &t : th_) t.join();
-  }
-  void copy(void *dst, const void *src, size_t n) {
-    const int parts = (int)th_.size() + 1;
-    if (parts == 1 || n < (size_t(64) << 10)) {
-      std::memcpy(dst, src, n);
-      return;
-    }
-    dst_ = static_cast<char *>(dst);
-    src_ = static_cast<const char *>(src);
-    n_ = n;
-    left_.store((int)th_.size(), std::memory_order_relaxed);
-    {
-      std::lock_guard<std::mutex> lk(mu_);
-      gen_.fetch_add(1, std::memory_order_release);
-    }
-    cv_.notify_all();
-    part((int)th_.size(), parts);
-    // the workers' parts are as large as the one just done
-    while (left_.load(std::memory_order_acquire) != 0) std::this_thread::yield();
-  }
-
- private:
-  void part(int k, int parts) {
-    const size_t page = 4096, per = (n_ / parts + page - 1) / page * page, at = per * k;
-    if (at >= n_) return;
-    std::memcpy(dst_ + at, src_ + at, (k == parts - 1 || at + per > n_) ? n_ - at : per);
-  }
-  void work(int k) {
-    unsigned seen = 0;
-    for (;;) {
-      // chunks of one transfer follow each other within microseconds: look
-      // for the next one a while before sleeping
-      for (int spin = 0; spin < 4000 && gen_.load(std::memory_order_acquire) == seen; spin++) std::this_thread::yield();
-      if (gen_.load(std::memory_order_acquire) == seen) {
-        std::unique_lock<std::mutex> lk(mu_);
-        cv_.wait(lk, [&] { return gen_.load(std::memory_order_acquire) != seen; });
-      }
-      seen = gen_.load(std::memory_order_acquire);
-      if (quit_) return;
-      part(k, (int)th_.size() + 1);
-      left_.fetch_sub(1, std::memory_order_release);
-    }
-  }
-  std::vector<std::thread> th_;
-  std::mutex mu_;
-  std::condition_variable cv_;
-  std::atomic<unsigned> gen_{0};
-  std::atomic<int> left_{0};
-  bool quit_ = false;
-  char *dst_ = nullptr;
-  const char *src_ = nullptr;
-  size_t n_ = 0;
-};
-
 // the cores this process may run on (its affinity mask, which containers set)
 int usable_cores() {
   cpu_set_t set;
@@ -125,7 +53,7 @@ struct Stager {
   std::mutex busy;
   char *ring = nullptr;
   cudaEvent_t ev[RING] = {};
-  std::unique_ptr<CopyPool> pool;
+  std::unique_ptr<CopyPool<>> pool;
   ~Stager() {
     if (ring)
       for (auto e : ev) cudaEventSynchronize(e);
@@ -137,11 +65,7 @@ struct Stager {
   bool ready() {
     if (ring) return true;
     const int cores = usable_cores();
-    try {
-      if (!pool) pool.reset(new CopyPool(cores >= 16 ? 7 : cores >= 4 ? cores / 2 - 1 : 0));
-    } catch (const std::exception &) {
-      return false;  // no threads: the driver's path
-    }
+    if (!pool) pool.reset(new CopyPool<>(cores >= 16 ? 7 : cores >= 4 ? cores / 2 - 1 : 0));
     for (auto &e : ev)
       if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
         cudaGetLastError();
