@@ -16,11 +16,14 @@
 // belong to one device; they are made by the first copy that needs them,
 // shared by every lattice of the device and given back when the last lattice
 // goes.  One transfer uses them at a time: a second thread's transfer that
-// finds them busy takes the driver's path.
+// finds them busy takes the driver's path, and so do all for a while after a
+// copy thread lost its core in the middle of a copy (CopyPool::crowded).
 #include "host_copy.h"
 
 #include <sched.h>
 
+#include <algorithm>
+#include <cstdio>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -41,12 +44,20 @@ constexpr int RING = 8;
 // below this the driver's path is as fast (one chunk, no overlap)
 constexpr size_t SMALLEST = size_t(256) << 10;
 
-// the cores this process may run on (its affinity mask, which containers set)
+// the cores this process may run on: its affinity mask and its CPU quota
+// (cgroup v2), either of which a container may set
 int usable_cores() {
+  int n = (int)std::thread::hardware_concurrency();
   cpu_set_t set;
   CPU_ZERO(&set);
-  if (sched_getaffinity(0, sizeof(set), &set) == 0) return CPU_COUNT(&set);
-  return (int)std::thread::hardware_concurrency();
+  if (sched_getaffinity(0, sizeof(set), &set) == 0) n = CPU_COUNT(&set);
+  if (FILE *f = std::fopen("/sys/fs/cgroup/cpu.max", "r")) {
+    long quota = 0, period = 0;  // "max 100000" without a limit
+    if (std::fscanf(f, "%ld %ld", &quota, &period) == 2 && quota > 0 && period > 0)
+      n = std::min(n, (int)std::max(1L, quota / period));
+    std::fclose(f);
+  }
+  return n;
 }
 
 struct Stager {
@@ -66,6 +77,7 @@ struct Stager {
     if (ring) return true;
     const int cores = usable_cores();
     if (!pool) pool.reset(new CopyPool<>(cores >= 16 ? 7 : cores >= 4 ? cores / 2 - 1 : 0));
+    if (pool->workers() == 0) return false;
     for (auto &e : ev)
       if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
         cudaGetLastError();
@@ -111,7 +123,7 @@ std::shared_ptr<Stager> take(const void *host, size_t bytes, std::unique_lock<st
   std::shared_ptr<Stager> s = stager_of(dev, false);
   if (!s) return nullptr;
   lk = std::unique_lock<std::mutex>(s->busy, std::try_to_lock);
-  if (!lk.owns_lock() || !s->ready()) {
+  if (!lk.owns_lock() || !s->ready() || s->pool->crowded()) {
     if (lk.owns_lock()) lk.unlock();
     return nullptr;
   }
