@@ -143,12 +143,12 @@ struct MobiusPlan {
   double coef = 0.0;
 };
 
-// A packed pair of real mixing matrices as out = a x + g y with y a shift of
+// A packed pair of real mixing matrices as out = d x + e y with y a shift of
 // x (BAND) or a recurrence along the slices (SCAN), per chirality (mix_scan.cu)
 struct MixScan {
   enum { DENSE = 0, SCAN = 1, BAND = 2 };
   int kind = DENSE;
-  double rho[2], w[2], a[2], g[2];
+  double rho[2], w[2], d[2], e[2];
   int down[2];  // 1: the recurrence starts at the last slice
 };
 MixScan fit_mix_scan(int ls, const std::vector<double> &packed);

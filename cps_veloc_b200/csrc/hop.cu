@@ -55,7 +55,7 @@ void launch_hop(const Dirac &D, const HopLaunch &L, const SpinorView &in, const 
   if (scan) {
     hp.scan = scan->kind;
     for (int c = 0; c < 2; c++) {
-      const double v[4] = {scan->rho[c], scan->w[c], scan->a[c], scan->g[c]};
+      const double v[4] = {scan->rho[c], scan->w[c], scan->d[c], scan->e[c]};
       hp.scan_down[c] = scan->down[c];
       for (int k = 0; k < 4; k++) {
         hp.scan_d[c][k] = v[k];

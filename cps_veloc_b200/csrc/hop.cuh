@@ -90,7 +90,7 @@ struct HopParams {
   const double *mix;    // [2][ls][ls] row-major, upper then lower chirality ([..][re, im] if mix_cplx)
   int mix_cplx;         // complex mixing matrices (zMobius)
   // the two-term form of the mixing (MixScan; mix_scan.cu), per chirality:
-  // rho, w, a, g in the arithmetic precisions
+  // rho, w, d, e in the arithmetic precisions
   int scan;
   int scan_down[2];
   double scan_d[2][4];
@@ -509,7 +509,7 @@ __device__ __forceinline__ void mix_scan_epilogue(const HopParams &hp, int s, bo
   for (int q = tid; q < 12 * bx; q += nthr) {
     const int c = q >= 6 * bx;
     const R *cf = Q::coef(hp, c);
-    const R rho = cf[0], w = cf[1], a = cf[2], g = cf[3];
+    const R rho = cf[0], w = cf[1], d = cf[2], e = cf[3];
     const int step = hp.scan_down[c] ? -12 * bx : 12 * bx;
     T *col = sm + q + (hp.scan_down[c] ? (n - 1) * 12 * bx : 0);
     const T x0 = col[0];
@@ -518,20 +518,20 @@ __device__ __forceinline__ void mix_scan_epilogue(const HopParams &hp, int s, bo
       y = Q::mul(w, col[(n - 1) * step]);
       for (int k = 0; k < n; k++) {
         x = col[k * step];
-        col[k * step] = Q::fma(g, y, Q::mul(a, x));
+        col[k * step] = Q::fma(e, y, Q::mul(d, x));
         y = x;
       }
     } else {
       T h = x0;
 #pragma unroll 4
       for (int k = 1; k < n; k++) h = Q::fma(rho, h, col[k * step]);
-      y = Q::fma(w, h, x0);
-      col[0] = Q::fma(g, y, Q::mul(a, x0));
+      y = Q::mul(w, h);
+      col[0] = Q::fma(e, y, Q::mul(d, x0));
 #pragma unroll 4
       for (int k = 1; k < n; k++) {
-        x = col[k * step];
         y = Q::fma(rho, y, x);
-        col[k * step] = Q::fma(g, y, Q::mul(a, x));
+        x = col[k * step];
+        col[k * step] = Q::fma(e, y, Q::mul(d, x));
       }
     }
   }

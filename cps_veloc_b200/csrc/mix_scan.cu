@@ -2,17 +2,26 @@
 //
 // With the same real b, c on every slice all matrices of the Mobius operator
 // are functions of one shift S (slice s from s-1, the wall weighted -m, or
-// its mirror image from s+1): either B = a + g S (zmobius_dslash_4's mixing,
+// its mirror image from s+1): either B = d + e S (zmobius_dslash_4's mixing,
 // 1 + K D5) or a + g (1 + K S)^-1 (M5^-1, B M5^-1 and the products with
-// kappa_b, their adjoints, the MIT forms).  So out = a x + g y with
+// kappa_b, their adjoints, the MIT forms).  So out = d x + e y with
 //   band:  y_0 = w x_{n-1},        y_s = x_{s-1}
-//   scan:  h = sum_t rho^(n-1-t) x_t (Horner),  y_0 = x_0 + w h,
-//          y_s = rho y_{s-1} + x_s
-// (rho = -K, w = K m / (1 - K m rho^(n-1)), zmobius_m5inv.C:247-396 solves the
-// same bidiagonal-plus-corner system): 4 multiply-adds per real whatever Ls
-// is, where the dense matrix takes Ls.  fit_mix_scan recognises the form in
-// the packed matrices; what does not have it (slices with different real
-// b_s, c_s, complex ones, |K| > 1, Ls < 3) keeps the dense kernels.
+//   scan:  h = sum_t rho^(n-1-t) x_t (Horner),  y_0 = w h,
+//          y_s = rho y_{s-1} + x_{s-1}
+// (rho = -K; zmobius_m5inv.C:247-396 solves the same bidiagonal-plus-corner
+// system): 4 multiply-adds per real whatever Ls is, where the dense matrix
+// takes Ls.  d = a + g and e = g rho are of the size of the matrix; a and g
+// alone are not (B M5^-1 has a = c / K, 21 at b = 1.5, c = 0.5, M5 = 1.8 for
+// entries up to 1.5), so a sum of a x and g y would cancel.
+//
+// fit_mix_scan recognises the form in the packed matrices; what does not have
+// it (slices with different real b_s, c_s, complex ones, |K| > 0.6, Ls < 3)
+// keeps the dense kernels.  Error of one mixing in the 2-norm, of the exact
+// one, dense / this, 6 <= Ls <= 32, 0.001 <= m <= 0.5: FP32 2.5e-8 - 1.5e-7 /
+// 2.5e-8 - 1.1e-7, FP64 6e-17 - 2.8e-16 / 5e-17 - 1.6e-16, and matrix by
+// matrix up to |K| = 0.6 at most 1.2 times the dense one's, 0.6 times in the
+// mean; from 0.65 on single ones reach 1.3 times, at 0.85 2 times (rho^k
+// carries k roundings of rho).
 //
 // FP64, FP32: a thread per 16-byte group of one site holds its Ls values in
 // registers (all loads in flight at once), so each field is read and written
@@ -35,7 +44,7 @@ namespace {
 
 // coefficients of one chirality in the arithmetic precision
 template <typename R> struct ScanCoef {
-  R rho, w, a, g;
+  R rho, w, d, e;
   int down;
 };
 template <typename R> struct ScanArg {
@@ -84,12 +93,12 @@ __global__ void __launch_bounds__(SCAN_SITES * PrecTraits<P>::NG)
       T h = x[0];
 #pragma unroll
       for (int k = 1; k < LS; k++) h = fma2(c.rho, h, x[k]);
-      y = fma2(c.w, h, x[0]);
+      y = mul2(c.w, h);
     }
 #pragma unroll
     for (int k = 0; k < LS; k++) {
-      op[k * step] = fma2(c.g, y, mul2(c.a, x[k]));
-      if (k + 1 < LS) y = BAND ? x[k] : fma2(c.rho, y, x[k + 1]);
+      op[k * step] = fma2(c.e, y, mul2(c.d, x[k]));
+      if (k + 1 < LS) y = BAND ? x[k] : fma2(c.rho, y, x[k]);
     }
   } else {
     T y;
@@ -100,13 +109,13 @@ __global__ void __launch_bounds__(SCAN_SITES * PrecTraits<P>::NG)
       T h = x0;
 #pragma unroll 4
       for (int k = 1; k < n; k++) h = fma2(c.rho, h, __ldg(ip + k * step));
-      y = fma2(c.w, h, x0);
+      y = mul2(c.w, h);
     }
     T x = x0;
     for (int k = 0; k < n; k++) {
       const T xn = k + 1 < n ? __ldg(ip + (k + 1) * step) : x;
-      op[k * step] = fma2(c.g, y, mul2(c.a, x));
-      y = BAND ? x : fma2(c.rho, y, xn);
+      op[k * step] = fma2(c.e, y, mul2(c.d, x));
+      y = BAND ? x : fma2(c.rho, y, x);
       x = xn;
     }
   }
@@ -128,8 +137,10 @@ __device__ __forceinline__ void unpack12(const Half12 &v, int lower, float2 (&f)
   for (int k = 0; k < 6; k++) f[k] = __half22float2(*reinterpret_cast<const __half2 *>(&w[k]));
 }
 
+// (the blocks per SM hold the registers where the loads in flight need them:
+// at Ls = 12 two blocks instead of three take 132 us instead of 109, 24^3x64)
 template <int LS, bool BAND>
-__global__ void __launch_bounds__(SCAN_HALF_TPB)
+__global__ void __launch_bounds__(SCAN_HALF_TPB, LS <= 8 ? 4 : LS <= 12 ? 3 : 2)
     scan_half_kernel(SpinorView in, SpinorView out, const ScanArg<float> arg, const SolverScalars *st, int gate, int rev) {
   if (gate == GATE_RUNNING && st[blockIdx.z].done) return;
   if (gate == GATE_RELIABLE && (st[blockIdx.z].done || !st[blockIdx.z].reliable)) return;
@@ -166,8 +177,8 @@ __global__ void __launch_bounds__(SCAN_HALF_TPB)
 #pragma unroll
     for (int q = 0; q < 6; q++) f[q] = __fmul2_rn(f[q], make_float2(nrm[k], nrm[k]));
   };
-  const float2 rho = make_float2(c.rho, c.rho), w = make_float2(c.w, c.w), a = make_float2(c.a, c.a),
-               gg = make_float2(c.g, c.g);
+  const float2 rho = make_float2(c.rho, c.rho), w = make_float2(c.w, c.w), d = make_float2(c.d, c.d),
+               e = make_float2(c.e, c.e);
   float2 y[6], v[6];
   if constexpr (BAND) {
     value(LS - 1, v);
@@ -183,11 +194,11 @@ __global__ void __launch_bounds__(SCAN_HALF_TPB)
 #pragma unroll
       for (int q = 0; q < 6; q++) h[q] = __ffma2_rn(rho, h[q], v[q]);
     }
-    value(0, v);
 #pragma unroll
-    for (int q = 0; q < 6; q++) y[q] = __ffma2_rn(w, h[q], v[q]);
+    for (int q = 0; q < 6; q++) y[q] = __fmul2_rn(w, h[q]);
+    value(0, v);
   }
-  // out = a x + g y; its norm needs the other chirality's maximum for the same
+  // out = d x + e y; its norm needs the other chirality's maximum for the same
   // slice, and the two recurrences run through the slices from opposite ends:
   // at step k one is at slice k, the other at LS-1-k.  So the first half of
   // the outputs waits in registers, and step k of the second half finishes
@@ -212,12 +223,17 @@ __global__ void __launch_bounds__(SCAN_HALF_TPB)
   float mk[LS / 2];
 #pragma unroll
   for (int k = 0; k < LS; k++) {
+    if (k > 0) value(k, v);
     float2 o[6];
     float m = 0.f;
 #pragma unroll
     for (int q = 0; q < 6; q++) {
-      o[q] = __ffma2_rn(gg, y[q], __fmul2_rn(a, v[q]));
+      o[q] = __ffma2_rn(e, y[q], __fmul2_rn(d, v[q]));
       m = fmaxf(m, fmaxf(fabsf(o[q].x), fabsf(o[q].y)));
+    }
+    if (k + 1 < LS) {
+#pragma unroll
+      for (int q = 0; q < 6; q++) y[q] = BAND ? v[q] : __ffma2_rn(rho, y[q], v[q]);
     }
     if (k < LS / 2) {
 #pragma unroll
@@ -226,28 +242,17 @@ __global__ void __launch_bounds__(SCAN_HALF_TPB)
     } else if (2 * k + 1 == LS) {  // the middle slice of an odd Ls: both are there
       finish(k, o, fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16)));
     } else {
-      const int e = LS - 1 - k;
-      const float other_now = __shfl_xor_sync(0xffffffffu, m, 16), other_kept = __shfl_xor_sync(0xffffffffu, mk[e], 16);
+      const int q = LS - 1 - k;
+      const float other_now = __shfl_xor_sync(0xffffffffu, m, 16), other_kept = __shfl_xor_sync(0xffffffffu, mk[q], 16);
       finish(k, o, fmaxf(m, other_kept));
-      finish(e, keep[e], fmaxf(mk[e], other_now));
-    }
-    if (k + 1 < LS) {
-      if constexpr (BAND) {
-#pragma unroll
-        for (int q = 0; q < 6; q++) y[q] = v[q];
-        value(k + 1, v);
-      } else {
-        value(k + 1, v);
-#pragma unroll
-        for (int q = 0; q < 6; q++) y[q] = __ffma2_rn(rho, y[q], v[q]);
-      }
+      finish(q, keep[q], fmaxf(mk[q], other_now));
     }
   }
 }
 
 template <typename R> ScanArg<R> scan_arg(const MixScan &m) {
   ScanArg<R> a;
-  for (int k = 0; k < 2; k++) a.c[k] = {R(m.rho[k]), R(m.w[k]), R(m.a[k]), R(m.g[k]), m.down[k]};
+  for (int k = 0; k < 2; k++) a.c[k] = {R(m.rho[k]), R(m.w[k]), R(m.d[k]), R(m.e[k]), m.down[k]};
   return a;
 }
 
@@ -274,39 +279,22 @@ void launch_half(const MixScan &m, const SpinorView &in, const SpinorView &out, 
 // one chirality; m(i, j) the matrix seen from the end the recurrence starts at
 template <typename F>
 bool fit(int n, F &&m, double scale, MixScan &s, int c, int down, int kind) {
-  const double tol = 1e-14 * scale;
-  auto same = [&](auto &&model) {
-    for (int i = 0; i < n; i++)
-      for (int j = 0; j < n; j++)
-        if (!(std::fabs(m(i, j) - model(i, j)) <= tol)) return false;
-    return true;
-  };
-  const double d1 = m(1, 0), corner = m(0, n - 1);
-  if (kind == MixScan::BAND) {
-    if (d1 == 0.0) return false;
-    const double a = m(0, 0);
-    if (!same([&](int i, int j) { return i == j ? a : i == j + 1 ? d1 : (i == 0 && j == n - 1) ? corner : 0.0; })) return false;
-    s.rho[c] = 0.0;
-    s.w[c] = corner / d1;
-    s.a[c] = a;
-    s.g[c] = d1;
-  } else {
-    const double d2 = m(2, 0);
-    if (d1 == 0.0 || d2 == 0.0) return false;
-    const double rho = d2 / d1;
-    if (!(std::fabs(rho) <= 1.0)) return false;
-    const double g = d1 / rho - corner * std::pow(rho, n - 1);
-    if (g == 0.0) return false;
-    const double w = corner / g, a = m(0, 0) - g * (1.0 + w * std::pow(rho, n - 1));
-    if (!same([&](int i, int j) {
-          return (i == j ? a : 0.0) + g * ((i >= j ? std::pow(rho, i - j) : 0.0) + w * std::pow(rho, n - 1 - j + i));
-        }))
-      return false;
-    s.rho[c] = rho;
-    s.w[c] = w;
-    s.a[c] = a;
-    s.g[c] = g;
-  }
+  const double tol = 1e-15 * scale;  // some roundings of the matrix product it came from
+  const double corner = m(0, n - 1), d1 = m(1, 0);
+  const double rho = kind == MixScan::BAND ? 0.0 : m(2, 0) / d1;
+  if (d1 == 0.0 || !(std::fabs(rho) <= 0.6) || (kind == MixScan::SCAN && rho == 0.0)) return false;
+  const double e = d1 - corner * std::pow(rho, n), w = corner / e, d = m(0, 0) - corner * std::pow(rho, n - 1);
+  if (!std::isfinite(w)) return false;
+  // (pow(0, 0) is 1)
+  for (int i = 0; i < n; i++)
+    for (int j = 0; j < n; j++) {
+      const double model = (i == j ? d : 0.0) + e * ((i > j ? std::pow(rho, i - 1 - j) : 0.0) + w * std::pow(rho, n - 1 - j + i));
+      if (!(std::fabs(m(i, j) - model) <= tol)) return false;
+    }
+  s.rho[c] = rho;
+  s.w[c] = w;
+  s.d[c] = d;
+  s.e[c] = e;
   s.down[c] = down;
   return true;
 }
