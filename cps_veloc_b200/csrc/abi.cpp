@@ -1526,6 +1526,7 @@ int cpsgpu_set_mix_impl(cpsgpu_dirac d, int impl) {
     if (impl < 0 || impl > 3)
       throw Error(CPSGPU_ERR_ARG, "mixing kernel: 0 default, 1 tensor cores, 2 shared memory, 3 register-tiled");
     CPSGPU_CUDA(cudaStreamSynchronize(d->D->lat->stream));
+    d->D->mix_named = (impl == 2 || impl == 3);
     d->D->mix_tc = (impl == 1);
     d->D->mix_reg = (impl != 2);
     d->D->mix_bulk = (impl == 0 || impl == 1);

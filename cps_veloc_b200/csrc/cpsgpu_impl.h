@@ -225,9 +225,10 @@ struct Dirac {
   std::unordered_map<const void *, std::vector<double>> mix_host;
   // ... and its two-term form, where it has one
   std::unordered_map<const void *, MixScan> mix_scan;
+  // (null when the caller has named a dense kernel)
   const MixScan *scan_of(const void *mix) const {
     const auto it = mix_scan.find(mix);
-    return it == mix_scan.end() ? nullptr : &it->second;
+    return (mix_named || it == mix_scan.end()) ? nullptr : &it->second;
   }
   // remember the host form of a real matrix just uploaded at ptr
   void keep_mix(const void *ptr, const std::vector<double> &h) {
@@ -242,6 +243,9 @@ struct Dirac {
   // right-hand sides per hop tile (consecutive blocks share links across
   // this many solves), per precision, set by the autotuner; 0 = untuned
   int rtile[3] = {0, 0, 0};
+  // cpsgpu_set_mix_impl named a dense mixing kernel: no recurrences, the
+  // hop's mixing epilogue dense too
+  bool mix_named = false;
   // the standalone Ls x Ls mixings of FP16 fields on the tensor cores
   // (mix_tc.cu) instead of the CUDA cores
   bool mix_tc = false;

@@ -637,15 +637,17 @@ class DiracOpMobius(_DiracOp):
         return v.value
 
     MIX_DEFAULT, MIX_TENSOR_CORES, MIX_SHARED, MIX_REG = 0, 1, 2, 3
-    MIX_BULK = MIX_DEFAULT  # FP16 fields: staged by bulk copies where it applies
+    MIX_BULK = MIX_DEFAULT  # FP16 fields, b_s and c_s that differ between slices: staged by bulk copies where it applies
 
     def set_mix_impl(self, impl) -> None:
-        """the kernel of the standalone Ls x Ls mixings: MIX_DEFAULT (0: FP16
-        fields the register-tiled arithmetic on input tiles staged by bulk
-        asynchronous copies, else as MIX_REG), MIX_TENSOR_CORES (1, FP16
-        fields on the tensor cores), MIX_SHARED (2, the shared-memory
-        CUDA-core kernel) or MIX_REG (3, register-tiled CUDA cores);
-        True / False mean 1 / 0"""
+        """the kernel of the standalone Ls x Ls mixings: MIX_DEFAULT (0: the
+        recurrence along the slices where b, c are real and the same on every
+        slice, in the hop's mixing epilogue too; else FP16 fields the
+        register-tiled arithmetic on input tiles staged by bulk asynchronous
+        copies, and what that does not cover as MIX_REG), MIX_TENSOR_CORES
+        (1, FP16 fields on the tensor cores), MIX_SHARED (2, the
+        shared-memory CUDA-core kernel) or MIX_REG (3, register-tiled CUDA
+        cores), the last two for every matrix; True / False mean 1 / 0"""
         impl = int(impl) if not isinstance(impl, bool) else (1 if impl else 0)
         check(lib().cpsgpu_set_mix_impl(self._h, impl))
 

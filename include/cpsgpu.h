@@ -231,10 +231,14 @@ int cpsgpu_dirac_set_pc_type(cpsgpu_dirac d, int pc_type);
 int cpsgpu_dirac_get_pc_type(cpsgpu_dirac d, int *pc_type);
 /* No counterpart in the reference: the kernel of the Mobius operator's
  * standalone Ls x Ls mixings (M5^-1, the first step of MatPc).
- *   0 (the default): for FP16 fields the register-tiled arithmetic of 3 on
- *     input tiles staged in shared memory by bulk asynchronous copies, two
- *     stages per persistent block (mix_bulk.cu; Ls 8, 10, 12, 16, sites per
- *     checkerboard slice a multiple of 32, real b, c), else as 3;
+ *   0 (the default): matrices of one real b, c on every slice (|K| <= 0.6,
+ *     Ls >= 3) as a recurrence along the slices (mix_scan.cu), here and in
+ *     the hop's mixing epilogue; for the others (and, at FP16, the Ls that
+ *     mix_scan.cu does not instantiate), FP16 fields the register-tiled
+ *     arithmetic of 3 on input tiles staged in shared memory by bulk
+ *     asynchronous copies, two stages per persistent block (mix_bulk.cu;
+ *     Ls 8, 10, 12, 16, sites per checkerboard slice a multiple of 32, real
+ *     b_s, c_s), else as 3;
  *   1: for FP16 fields, mma.sync m16n8k16 contractions on the tensor cores
  *     (FP16 operands with the matrix split into high and low parts, FP32
  *     accumulation, mix_tc.cu; Ls <= 16, real b, c), else as 0;
@@ -245,11 +249,9 @@ int cpsgpu_dirac_get_pc_type(cpsgpu_dirac d, int *pc_type);
  *     the two real matrices are a kernel parameter, every thread computes
  *     all Ls output slices of a block of reals with packed FP32 multiply-adds
  *     (Ls 8, 10, 12, 16, 20, 24; real b, c); FP64 fields as 2.
- * Matrices of one real b, c on every slice (|K| <= 1, Ls >= 3) run as a
- * recurrence along the slices under 0, 2 and 3 alike (mix_scan.cu); the
- * kernels named above then apply to the others (real b_s, c_s that differ
- * between slices, and at FP16 the Ls that mix_scan.cu does not instantiate).
- * Every form but 1 gives the same bits. */
+ * 2 and 3 run their dense kernels for every matrix, the hop's mixing
+ * epilogue too, and give the same bits; so does 0 for the matrices that are
+ * no recurrence. */
 int cpsgpu_set_mix_impl(cpsgpu_dirac d, int impl);
 
 /* ---- solvers ---- */

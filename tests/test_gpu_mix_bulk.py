@@ -1,7 +1,7 @@
-"""The bulk-copy staged Ls x Ls mixing kernel (mix_bulk.cu, cpsgpu_set_mix_impl
-3: FP16 fields, real b, c, Ls 8, 10, 12, 16, sites per checkerboard slice a
-multiple of 32) against the register-tiled kernel whose arithmetic it
-repeats: the same bits for M5^-1 and its dagger, MatPc, MatPcDag and
+"""The bulk-copy staged Ls x Ls mixing kernel (mix_bulk.cu, the default for
+FP16 fields with real b_s, c_s that differ between slices, Ls 8, 10, 12, 16,
+sites per checkerboard slice a multiple of 32) against the register-tiled
+kernel (cpsgpu_set_mix_impl 3) whose arithmetic it repeats: the same bits for M5^-1 and its dagger, MatPc, MatPcDag and
 MatPcDagMatPc, over lattices with one and with many 32-site tiles per slice
 (so every block of the persistent grid walks several tiles through both
 stages), a batched FP16-inner solve with its gated right-hand sides, and the
@@ -23,7 +23,14 @@ def _op(L, ls, seed):
     u = gen_gauge(L, seed=seed)
     lat = Lattice(L)
     lat.import_gauge(u)
-    return u, lat, DiracOpMobius(lat, mass=0.05, ls=ls, b=1.5, c=0.5)
+    D = DiracOpMobius(lat, mass=0.05, ls=ls, b=1.5, c=0.5)
+    D.set_zmobius(*_slices(ls))  # matrices that are no recurrence along the slices, which the default would take
+    return u, lat, D
+
+
+def _slices(ls):
+    b = [1.5 + 0.005 * s for s in range(ls)]  # (MatPcDag of such slices is nearly MatPc^dagger: the solve converges)
+    return b, [x - 1.0 for x in b]
 
 
 @pytest.mark.parametrize("L,ls", [((4, 4, 4, 4), 8), ((4, 4, 4, 8), 12), ((8, 8, 8, 8), 12), ((8, 8, 8, 16), 16),
@@ -40,6 +47,7 @@ def test_mix_bulk_bitwise_and_oracle(oracle, L, ls, prec):
     for a, b in zip(out[D.MIX_REG], out[D.MIX_BULK]):
         np.testing.assert_array_equal(a, b)
     ops = OracleOps(oracle, L, u, ls=ls, b=1.5, c=0.5)
+    ops.set_zmobius(*([complex(x) for x in v] for v in _slices(ls)))
     tol = {A.SINGLE: 2e-6, A.HALF: 5e-3}[prec]
     for dag in (0, 1):
         assert rel(out[D.MIX_BULK][dag], ops.mobius_m5inv(x, 0.05, dag)) < tol

@@ -1,6 +1,7 @@
-"""The register-tiled Ls x Ls mixing kernel (mix_reg.cu, the default for
-FP32 and FP16 fields with real b, c at Ls 8, 10, 12, 16, 20, 24) against the
-shared-memory kernel it replaced (cpsgpu_set_mix_impl 2) and the oracle.
+"""The register-tiled Ls x Ls mixing kernel (mix_reg.cu, cpsgpu_set_mix_impl
+3: FP32 and FP16 fields with real b, c at Ls 8, 10, 12, 16, 20, 24) against the
+shared-memory kernel (cpsgpu_set_mix_impl 2) and the oracle, both named: the
+default would take the recurrence along the slices.
 Both sum the Ls terms of every output in the same order with fused
 multiply-adds and store FP16 through the same norm rule, so every field
 they write is bit-identical: M5^-1 and its dagger, MatPc, MatPcDag and

@@ -92,3 +92,29 @@ def test_precision_of_the_form(oracle, b, c, ls):
     yo, _ = ops.mobius_mdagm(x, 0.05)
     assert rel(D.MatPcDagMatPc(x, prec=A.SINGLE)[0], yo) < 8e-7
     assert rel(D.MatPcDagMatPc(x, prec=A.DOUBLE)[0], yo) < 4e-15
+
+
+@pytest.mark.parametrize("prec", [A.DOUBLE, A.SINGLE, A.HALF])
+def test_named_kernels_are_dense(oracle, prec):
+    """cpsgpu_set_mix_impl 2 and 3 run the dense kernels on matrices that have the recurrence's form, in the standalone
+    mixings and the hop's epilogue: their bits are each other's and not the default's, and the default is no further
+    from the oracle (the roundings of one side may exceed the other's by chance: 1.3)"""
+    D, ops = _op(oracle, (4, 4, 4, 4), 12, 1.45, 0.45)
+    x = gen_gaussian(D.f_size, seed=962)
+
+    def fields():
+        return [D.M5inv(x, 0, prec=prec), D.M5inv(x, 1, prec=prec), D.Dslash4(x, 0, 1, prec=prec), D.MatPcDagMatPc(x, prec=prec)[0]]
+
+    default = fields()
+    D.set_mix_impl(D.MIX_SHARED)
+    shared = fields()
+    D.set_mix_impl(D.MIX_REG)
+    ref = [ops.mobius_m5inv(x, 0.05, 0), ops.mobius_m5inv(x, 0.05, 1), ops.mobius_dslash_4(x, 0.05, 0, 1),
+           ops.mobius_mdagm(x, 0.05)[0]]
+    for a, b, c, r in zip(fields(), shared, default, ref):
+        np.testing.assert_array_equal(a, b)
+        assert rel(c, r) <= 1.3 * rel(b, r)
+    assert any((b != c).any() for b, c in zip(shared, default))
+    D.set_mix_impl(D.MIX_DEFAULT)
+    for a, c in zip(fields(), default):
+        np.testing.assert_array_equal(a, c)
