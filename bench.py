@@ -372,13 +372,13 @@ def extra_mobius(A) -> dict:
            "speedup_vs_fp64_cg": r64.seconds / rh.seconds}
     for name, prec in (("fp64", A.DOUBLE), ("half", A.HALF)):
         ms, by = _dev_time(A, A.lib().cpsgpu_time_m5inv, D, prec, 20)
-        flops = 48 * ls * D.f_size // 24  # dense Ls x Ls, both chiralities
-        unit = ("CUDA cores, register-tiled (matrix as a kernel parameter), input tiles staged in shared "
-                "memory by bulk asynchronous copies" if prec == A.HALF else "CUDA cores, shared-memory staging")
         out[f"m5inv_{name}"] = {"ms": ms, "GB_s": by / ms / 1e6, "frac_of_measured_hbm": by / ms / 1e6 / pk,
-                                "flop_per_byte": flops / by, "unit": unit}
-        # the other CUDA-core kernels: shared-memory staging, register-tiled without bulk staging
+                                "flop_per_byte": 8 * D.f_size / by,  # four multiply-adds per real
+                                "unit": "CUDA cores, recurrence along the slices (the default for these b, c)"}
+        # the dense kernels, named: shared-memory staging, register-tiled (FP64: the shared-memory kernel again)
         for key, impl in (("shared_memory_kernel", D.MIX_SHARED), ("register_tiled_kernel", D.MIX_REG)):
+            if prec == A.DOUBLE and impl == D.MIX_REG:
+                continue
             D.set_mix_impl(impl)
             ms2, by2 = _dev_time(A, A.lib().cpsgpu_time_m5inv, D, prec, 20)
             out[f"m5inv_{name}_{key}"] = {"ms": ms2, "GB_s": by2 / ms2 / 1e6,
@@ -388,7 +388,8 @@ def extra_mobius(A) -> dict:
         A.check(A.lib().cpsgpu_time_dslash(D._h, prec, 1, 0, 20, C.byref(m2), C.byref(b2)))
         out[f"hop_{name}"] = {"ms": m2.value, "GB_s": b2.value / m2.value / 1e6}
     # the same M5^-1 of the FP16 field on the tensor cores (mma.sync m16n8k16),
-    # and the FP16-inner solve with every standalone mixing there
+    # and the FP16-inner solve with every standalone mixing there (the hop's
+    # mixing epilogue as by default)
     D.set_mix_impl(D.MIX_TENSOR_CORES)
     ms, by = _dev_time(A, A.lib().cpsgpu_time_m5inv, D, A.HALF, 20)
     out["m5inv_half_tensor_cores"] = {"ms": ms, "GB_s": by / ms / 1e6, "frac_of_measured_hbm": by / ms / 1e6 / pk,
@@ -400,7 +401,7 @@ def extra_mobius(A) -> dict:
     rt = D.InvCg(x, b, stop_rsd=STOP, max_num_iter=50000, precision=A.HALF)
     out["half_inner_cg_tensor_core_mixing"] = {"time_s": rt.seconds, "iterations": rt.iterations,
                                                "true_res": rt.true_res, "reliable_updates": rt.reliable_updates}
-    # and with the shared-memory mixing kernel, the form before the register-tiled one
+    # and with the dense mixings: the shared-memory kernel and the hop's dense epilogue
     D.set_mix_impl(D.MIX_SHARED)
     x = np.zeros(D.f_size)
     D.InvCg(x, b, stop_rsd=STOP, max_num_iter=50000, precision=A.HALF)
