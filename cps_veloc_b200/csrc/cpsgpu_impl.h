@@ -282,8 +282,12 @@ struct HopLaunch {
   const void *halo_fwd = nullptr, *halo_bwd = nullptr;  // t halos of a decomposed lattice (dd.cu)
   int sub = 0;  // HopSub: all sites, or (decomposed lattice) the interior or the two t-end slices
   double *partials = nullptr;  // the reduction's per-block partials (null: the lattice's buffer)
+  long beside = 0;  // 5D sites of other solves at work on the GPU at the same time (solve_batch)
   cudaGraphConditionalHandle *cond = nullptr;  // set by the finalize: this iteration's reliable update (one solve)
 };
+// does a hop without mixing take the four-threads-per-site kernel, unless the
+// caller has set its shape (hop.cu)
+bool hop_is_split(const Dirac &D, int prec, int nrhs, long beside);
 void launch_hop(const Dirac &D, const HopLaunch &L, const SpinorView &in, const SpinorView &out,
                 const SpinorView &x, const SpinorView &r, const SpinorView &sol, const SpinorView &p,
                 const SpinorView &b, SolverScalars *st);

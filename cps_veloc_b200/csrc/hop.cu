@@ -15,17 +15,26 @@ HopFn pick(int prec, const HopSel &q) {
   return prec == PREC_DOUBLE ? pick_hop_double(q) : prec == PREC_SINGLE ? pick_hop_single(q) : pick_hop_half(q);
 }
 
-// Launches of at most this many 5D sites (right-hand sides included) run four
-// threads per site (hop_split_kernel).  Microseconds per CG iteration without
-// / with, by sites: FP64 256 (Wilson 4^3x8) 41.7 / 28.1, 4096 (8^3x16) 40.9 /
-// 29.5, 16384 (DWF 8^4 Ls=8) 46.7 / 48.9, 32768 52.7 / 64.7; FP32 inner
-// solve 256 42.7 / 34.3, 16384 44.5 / 37.9, 32768 45.1 / 49.1; 8 right-hand
-// sides of 2048 sites FP64 46.8 / 48.6, FP32 48.6 / 40.5
+// At most this many 5D sites at work on the GPU (right-hand sides and the
+// other solves of a batch included) run four threads per site
+// (hop_split_kernel).  Microseconds per CG iteration without / with, by sites:
+// FP64 256 (Wilson 4^3x8) 37.2 / 24.7, 4096 (8^3x16) 41.2 / 31.7, 8192 (DWF
+// 8^3x4 Ls=8) 44.2 / 34.2, and with the kernel forced 16384 (8^4 Ls=8) 46.7 /
+// 48.9, 32768 52.7 / 64.7; FP32 inner solve 256 37.9 / 32.0, 4096 41.5 / 36.4,
+// 16384 41.9 / 38.3, forced 32768 45.1 / 49.1; FP16 inner solve 256 38.9 /
+// 32.8, 4096 43.1 / 39.4, 8192 45.3 / 42.1, 16384 43.2 / 40.4; 8 right-hand
+// sides of 2048 sites FP64 46.8 / 48.6, FP32 48.6 / 40.5.  A batch of 4 solves
+// of 16384 sites and 4 of 32768, FP32 inner: 12.8 ms, with the four threads in
+// the smaller ones 14.9
 constexpr long split_sites(int prec) { return prec == PREC_DOUBLE ? 8192 : 16384; }
 
 size_t real_size(int prec) { return prec == PREC_DOUBLE ? 8 : 4; }
 
 }  // namespace
+
+bool hop_is_split(const Dirac &D, int prec, int nrhs, long beside) {
+  return D.lat->t_nodes == 1 && D.lat->vh * D.ls * nrhs + beside <= split_sites(prec);
+}
 
 void launch_hop(const Dirac &D, const HopLaunch &L, const SpinorView &in, const SpinorView &out,
                 const SpinorView &x, const SpinorView &r, const SpinorView &sol, const SpinorView &p,
@@ -99,7 +108,7 @@ void launch_hop(const Dirac &D, const HopLaunch &L, const SpinorView &in, const 
   // block.z of a tuned shape: slices per thread (2: DWF slice pairs)
   const int ns = (block.z == 2 && hp.dwf && !mix && !halo && L.prec != PREC_DOUBLE && D.ls % (4 * (int)block.y) == 0) ? 2 : 1;
   block.z = 1;
-  const bool split_mu = !mix && !split && lat.vh * D.ls * in.nrhs <= split_sites(L.prec) && !hop_forced(key);
+  const bool split_mu = !mix && hop_is_split(D, L.prec, in.nrhs, L.beside) && !hop_forced(key);
   if (split_mu) block = dim3(SPLIT_BX, 1, 4);
   HopFn fn = pick(L.prec, HopSel{recon, L.ep, L.pr, L.px, L.dag != 0, ns, halo, split_mu});
   unsigned nsb;

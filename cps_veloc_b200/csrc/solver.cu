@@ -120,6 +120,7 @@ void CgSolver::emit_mdagm(int prec, const SpinorView &in, OpWork &w, int final_e
   Lh.prec = prec;
   Lh.gate = gate;
   Lh.partials = partials.as<double>();
+  Lh.beside = beside;
   // ---- M = MatPc ----
   Lh.dag = 0;
   SpinorView hop_in = w.t1.view(), x = in;
@@ -526,6 +527,18 @@ BatchGraph g_batch;
 void solve_batch(std::vector<CgSolver *> &solvers, const std::vector<CgArgs> &a,
                  std::vector<std::vector<CgResult>> &res) {
   const size_t n = solvers.size();
+  // while the batch is set up and runs, every solver's launches know of the others
+  struct Beside {
+    std::vector<CgSolver *> &v;
+    explicit Beside(std::vector<CgSolver *> &v_) : v(v_) {
+      long sites = 0;
+      for (CgSolver *S : v) sites += S->sites();
+      for (CgSolver *S : v) S->beside = sites - S->sites();
+    }
+    ~Beside() {
+      for (CgSolver *S : v) S->beside = 0;
+    }
+  } beside(solvers);
   std::vector<int> chunks(n);
   std::vector<unsigned long long> ids(n);
   for (size_t k = 0; k < n; k++) {

@@ -50,6 +50,8 @@ struct CgSolver {
   cudaStream_t side = nullptr;  // captures the conditional bodies
   DeviceBuffer ctl;              // the WHILE loop's body count and limit
   DeviceBuffer partials;         // this solver's reduction partials (solves may share a lattice)
+  long beside = 0;               // 5D sites of the solves whose loops run at the same time (solve_batch)
+  long sites() const { return D.lat->vh * D.ls * nrhs; }
   DeviceBuffer prm;              // begin_params: [nrhs][stop_rsd, shift]
   unsigned long long id = 0;     // new at every setup(): a graph holding this solver's buffers is current while it matches
   // state of one run between begin() and end()

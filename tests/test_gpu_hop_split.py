@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 from cps_veloc_b200 import _abi as A
-from cps_veloc_b200.dirac import DiracOpDwf, DiracOpWilson, Lattice, gen_gauge, gen_gaussian
+from cps_veloc_b200.dirac import DiracOpDwf, DiracOpWilson, Lattice, gen_gauge, gen_gaussian, solve_batch
 from helpers import OracleOps, rel
 
 pytestmark = pytest.mark.gpu
@@ -69,3 +69,26 @@ def test_solves(prec, shift):
     sols = [np.zeros(D.f_size) for _ in srcs]
     for b, s, q in zip(srcs, sols, D.InvCgMulti(sols, srcs, stop_rsd=1e-10, precision=prec)):
         assert q.status == A.CONVERGED and rel(D.MatPcDagMatPc(s)[0], b) <= 1.01e-10
+
+
+@pytest.mark.parametrize("count", [2, 3])
+def test_batch_counts_all_its_sites(count):
+    """Independent solves in one launch: the rule goes by the sites of all of them.  Two FP64 systems of 4096 sites are
+    few enough for four threads per site, three are not: those give the bits of the one-thread hop of the same shape
+    (the four-threads kernel sums its dot products in another order)."""
+    res = []
+    for forced in (False, True):
+        A.check(A.lib().cpsgpu_finalize())
+        items = []
+        for k in range(count):
+            lat = Lattice((4, 4, 8, 8), (1, 1, 1, -1))
+            lat.import_gauge(gen_gauge((4, 4, 8, 8), seed=976 + k))
+            D = DiracOpDwf(lat, mass=0.05, ls=8)
+            if forced:
+                D.set_hop_shape(A.DOUBLE, *D.hop_shape(A.DOUBLE))
+            items.append((D, np.zeros(D.f_size), gen_gaussian(D.f_size, seed=980 + k)))
+        for r in solve_batch(items, stop_rsd=1e-10, precision=A.DOUBLE):
+            assert r.status == A.CONVERGED and r.true_res <= 1e-10
+        res.append([sol for _, sol, _ in items])
+    assert all((a == b).all() for a, b in zip(*res)) == (count == 3)
+    A.check(A.lib().cpsgpu_finalize())
