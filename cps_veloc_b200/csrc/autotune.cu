@@ -5,7 +5,10 @@
 // hop, and the four fastest in each order on a whole MatPcDagMatPc, whose
 // epilogue kernels take the same shape; the mixing epilogue of the Mobius
 // operator needs all slices of a site in one block, so only its site count
-// varies.
+// varies.  A launch small enough for the four-threads-per-site kernel
+// (hop_is_split) takes that whatever the shape: then the link form alone is
+// timed, and the shapes, which larger lattices and batches share, stay as
+// they are.
 #include <algorithm>
 #include <vector>
 
@@ -52,6 +55,7 @@ int autotune(Dirac &D, int prec, int nrhs) {
   if (prec == PREC_DOUBLE) recons.push_back(L.recon(prec));
   else if (prec == PREC_HALF) recons = {12, 18, LINK_F32_12, LINK_F32_18};
   else recons = {12, 18};
+  const bool split = hop_is_split(D, prec, nrhs, 0);
   float best_recon_t = 1e30f;
   int best_recon = recons[0];
   for (int recon : recons) {
@@ -74,6 +78,7 @@ int autotune(Dirac &D, int prec, int nrhs) {
         }
     TuneKey key{prec, recon, EP_STORE, D.kind, D.ls};
     std::vector<std::pair<float, dim3>> timed;
+    if (split) cand.clear();
     for (auto b : cand) {
       tune_set(key, b);
       timed.push_back({time_launch(D, Lh, in, out, x, nullptr, e0, e1), b});
@@ -121,6 +126,19 @@ int autotune(Dirac &D, int prec, int nrhs) {
       CPSGPU_CUDA(cudaEventElapsedTime(&ms, e0, e1));
       return ms;
     };
+    if (split) {
+      // a shape set by the caller stays for the larger launches only
+      for (int ep : eps) {
+        const TuneKey k{prec, recon, ep, D.kind, D.ls};
+        if (hop_forced(k)) tune_set(k, hop_block(k, false), hop_order(k));
+      }
+      const float t = mdagm_ms();
+      if (t < best_recon_t) {
+        best_recon_t = t;
+        best_recon = recon;
+      }
+      continue;
+    }
     dim3 bestb = timed.empty() ? hop_block(key, false) : timed[0].second;
     int besto = ORDER_SLICES;
     if (L.t_nodes > 1) {

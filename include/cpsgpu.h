@@ -610,7 +610,9 @@ int cpsgpu_solve_batch(int n, const cpsgpu_dirac *ops, const cpsgpu_field *sol, 
 /* ---- tuning ---- */
 /* Time candidate block shapes of every hop kernel the operator uses, at
  * precision prec, and keep the fastest; with nrhs > 1 also the right-hand-
- * side tile.  Returns the number of tuned keys. */
+ * side tile.  Returns the number of tuned keys: no shapes where every launch
+ * is small enough for the four-threads-per-site kernel (below), whose shape
+ * is fixed. */
 int cpsgpu_autotune(cpsgpu_dirac d, int prec, int nrhs, int *tuned);
 /* Right-hand-side tile of batched hops at precision prec (no counterpart in
  * the reference): consecutive thread blocks apply the same links to `tile`
@@ -626,10 +628,12 @@ int cpsgpu_set_rhs_tile(cpsgpu_dirac d, int prec, int tile);
  * links), and the site order in which the grid's blocks take the lattice:
  * CPSGPU_ORDER_SLICES (consecutive blocks: every slice group of one block
  * of sites) or CPSGPU_ORDER_SITES (consecutive blocks: the site blocks of
- * one slice group, lexicographically).  get returns the shape in use; set
- * overrides the autotuner (and the four-threads-per-site kernel that small
- * launches of any other shape run).  The shape table (like the autotuner's) is shared by every
- * operator of the same kind, Ls, precision and link form. */
+ * one slice group, lexicographically).  The shape table (like the
+ * autotuner's) is shared by every operator of the same kind, Ls, precision
+ * and link form.  get returns the table's shape.  Small launches (at most
+ * 8192 5D sites at work on the GPU in FP64, 16384 in FP32 and FP16) run a
+ * kernel of four threads per site instead, unless the shape was set by set,
+ * which overrides the autotuner and that rule. */
 enum { CPSGPU_ORDER_SLICES = 0, CPSGPU_ORDER_SITES = 1 };
 int cpsgpu_get_hop_shape(cpsgpu_dirac d, int prec, int *sites, int *slices, int *slices_per_thread, int *order);
 int cpsgpu_set_hop_shape(cpsgpu_dirac d, int prec, int sites, int slices, int slices_per_thread, int order);
