@@ -205,6 +205,7 @@ int cpsgpu_finalize(void) {
   return guarded([&] {
     CPSGPU_CUDA(cudaDeviceSynchronize());
     tune_clear();
+    host_copy_finalize();
     return CPSGPU_OK;
   });
 }

@@ -83,8 +83,6 @@ enum DiracKind { KIND_WILSON = 0, KIND_DWF = 1, KIND_MOBIUS = 2 };
 
 struct EigenCacheDev;  // lowmode.cu
 
-struct HostCopyHold;  // host_copy.h
-
 struct Lattice {
   int L[4];
   long vh;
@@ -103,7 +101,6 @@ struct Lattice {
   DeviceBuffer partials;   // per-block reduction partials
   DeviceBuffer scratch_st; // SolverScalars for operator-only reductions
   double *pinned = nullptr;  // small pinned host buffer for scalars
-  HostCopyHold *host_copies = nullptr;  // the device's staging for pageable vectors
   std::vector<std::shared_ptr<EigenCacheDev>> eig_caches;  // named low-mode caches (lowmode.cu)
   int t_nodes = 1, t_coor = 0;  // t-slab decomposition: this lattice is slab t_coor of t_nodes (dd.cu)
   Lattice(const int L_[4], const double bc_[4]);

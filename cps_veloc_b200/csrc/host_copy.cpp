@@ -14,8 +14,11 @@
 //
 // The ring (RING chunks of at most CHUNK bytes, 16 MiB) and the threads
 // belong to one device; they are made by the first copy that needs them,
-// shared by every lattice of the device and given back when the last lattice
-// goes.  One transfer uses them at a time: a second thread's transfer that
+// shared by every lattice of the device and given back by cpsgpu_finalize.
+// They do not go with the last lattice: pinning the ring takes 6-9 ms, and a
+// program that makes a lattice per configuration would pay it each time
+// (an 8^4 lattice made, its links uploaded and closed: 6.7 ms, 18-22 with the
+// ring made and freed each time, 6.3 with the driver's path).  One transfer uses them at a time: a second thread's transfer that
 // finds them busy takes the driver's path, and so do all for a while after a
 // copy thread lost its core in the middle of a copy (CopyPool::crowded).
 #include "host_copy.h"
@@ -37,9 +40,8 @@ namespace cpsgpu {
 namespace {
 
 constexpr size_t CHUNK = size_t(2) << 20;
-// 8 x 4 MiB copies no faster and its pinning showed: making an 8^4 lattice and
-// uploading to it 31 ms, with 8 x 2 MiB 15; the force with 8 x 1 MiB 8.8 ms, with
-// 5 x 2 MiB 8.0, with 8 x 2 MiB 7.3
+// 8 x 4 MiB copies no faster; the force with 8 x 1 MiB 8.8 ms, with 5 x 2 MiB
+// 8.0, with 8 x 2 MiB 7.3
 constexpr int RING = 8;
 // below this the driver's path is as fast (one chunk, no overlap)
 constexpr size_t SMALLEST = size_t(256) << 10;
@@ -94,15 +96,13 @@ struct Stager {
 };
 
 std::mutex g_mu;
-std::map<int, std::weak_ptr<Stager>> g_stagers;
+// by device; never destroyed, as the CUDA runtime may be gone when statics are
+std::map<int, std::shared_ptr<Stager>> &g_stagers = *new std::map<int, std::shared_ptr<Stager>>;
 
-std::shared_ptr<Stager> stager_of(int device, bool make) {
+std::shared_ptr<Stager> stager_of(int device) {
   std::lock_guard<std::mutex> lk(g_mu);
-  std::shared_ptr<Stager> s = g_stagers[device].lock();
-  if (!s && make) {
-    s = std::make_shared<Stager>();
-    g_stagers[device] = s;
-  }
+  std::shared_ptr<Stager> &s = g_stagers[device];
+  if (!s) s = std::make_shared<Stager>();
   return s;
 }
 
@@ -120,8 +120,7 @@ std::shared_ptr<Stager> take(const void *host, size_t bytes, std::unique_lock<st
   if (bytes < SMALLEST || !pageable(host)) return nullptr;
   int dev = 0;
   CPSGPU_CUDA(cudaGetDevice(&dev));
-  std::shared_ptr<Stager> s = stager_of(dev, false);
-  if (!s) return nullptr;
+  std::shared_ptr<Stager> s = stager_of(dev);
   lk = std::unique_lock<std::mutex>(s->busy, std::try_to_lock);
   if (!lk.owns_lock() || !s->ready() || s->pool->crowded()) {
     if (lk.owns_lock()) lk.unlock();
@@ -138,12 +137,11 @@ size_t chunk_of(size_t bytes) {
 
 }  // namespace
 
-struct HostCopyHold {
-  std::shared_ptr<Stager> s;
-};
-
-HostCopyHold *host_copy_hold(int device) { return new HostCopyHold{stager_of(device, true)}; }
-void host_copy_release(HostCopyHold *h) { delete h; }
+void host_copy_finalize() {
+  std::map<int, std::shared_ptr<Stager>> gone;  // a transfer on another thread keeps its own until it ends
+  std::lock_guard<std::mutex> lk(g_mu);
+  gone.swap(g_stagers);
+}
 
 void copy_to_device(cudaStream_t stream, void *dst, const void *src, size_t bytes) {
   std::shared_ptr<Stager> s;  // outlives its lock

@@ -13,10 +13,8 @@ namespace cpsgpu {
 void copy_to_device(cudaStream_t stream, void *dst, const void *src, size_t bytes);
 void copy_to_host(cudaStream_t stream, void *dst, const void *src, size_t bytes);
 
-// Holds the device's staging buffers and copy threads alive (a Lattice does);
-// they are made by the first pageable copy and given back with the last holder.
-struct HostCopyHold;
-HostCopyHold *host_copy_hold(int device);
-void host_copy_release(HostCopyHold *h);
+// Gives back the staging buffers and copy threads (cpsgpu_finalize); the next
+// pageable copy makes them anew.
+void host_copy_finalize();
 
 }  // namespace cpsgpu

@@ -16,7 +16,6 @@
 #include <cstring>
 
 #include "cpsgpu_impl.h"
-#include "host_copy.h"
 #include "hop.cuh"
 
 namespace cpsgpu {
@@ -39,7 +38,6 @@ Lattice::Lattice(const int L_[4], const double bc_[4]) {
   own_stream = stream;
   CPSGPU_CUDA(cudaMallocHost(&pinned, 64 * sizeof(double)));
   scratch_st.alloc(sizeof(SolverScalars) * 4);
-  host_copies = host_copy_hold(device);
   CPSGPU_CUDA(cudaMemsetAsync(scratch_st.ptr, 0, scratch_st.bytes, stream));
 }
 
@@ -49,7 +47,6 @@ Lattice::~Lattice() {
     cudaStreamSynchronize(own_stream);
     cudaStreamDestroy(own_stream);
   }
-  host_copy_release(host_copies);
   if (pinned) cudaFreeHost(pinned);
 }
 
