@@ -101,6 +101,9 @@ struct Lattice {
   DeviceBuffer partials;   // per-block reduction partials
   DeviceBuffer scratch_st; // SolverScalars for operator-only reductions
   double *pinned = nullptr;  // small pinned host buffer for scalars
+  // the multishift's kept residuals, one buffer for all operators of the
+  // lattice (a call has the stream to itself), held by those that use it
+  std::weak_ptr<DeviceBuffer> ms_ring;
   std::vector<std::shared_ptr<EigenCacheDev>> eig_caches;  // named low-mode caches (lowmode.cu)
   int t_nodes = 1, t_coor = 0;  // t-slab decomposition: this lattice is slab t_coor of t_nodes (dd.cu)
   Lattice(const int L_[4], const double bc_[4]);
@@ -175,7 +178,7 @@ struct CachedGraph {
 struct MsWork {
   Field chi, r, tmp;
   std::vector<Field> p, psi;
-  std::vector<Field> ring;  // residuals of a chunk's iterations (deferred updates); the last is r
+  std::shared_ptr<DeviceBuffer> ring;  // residuals of a chunk's iterations (deferred updates; the last is r): Lattice::ms_ring
   DeviceBuffer st, ms, pv, psiv, partials;
   OpWork w;
   // The graphs hold the addresses of the buffers above: whichever of those is

@@ -432,36 +432,45 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
   // slot).  From 3 shifts on: with 2 the flush reads as much as it saves.
   // Seven more vectors beside the 2 n + 5 of the workspace, taken only while
   // they are a small part of the free memory; else every iteration updates
-  // every shift.  Measured, the
-  // whole call: n = 16 summed, Wilson 24^3x48 FP64, 63.3 -> 52.9 ms (12.6 ms
-  // of it upload); n = 10, DWF 12^3x24 Ls=8 FP64, 74.4 -> 54.0 ms (23 ms of
-  // it host copies)
+  // every shift.  One ring serves all operators of a lattice, goes with the
+  // last of them, and a large one goes with the call.  Measured, the whole
+  // call: n = 16 summed, Wilson 24^3x48 FP64, 63.3 -> 52.9 ms (12.6 ms of it
+  // upload); n = 10, DWF 12^3x24 Ls=8 FP64, 74.4 -> 54.0 ms (23 ms of it host
+  // copies)
+  constexpr size_t ring_kept = size_t(2) << 30;
+  const size_t ring_stride = (r.data.bytes + 255) & ~size_t(255), ring_bytes = (MS_DEFER - 1) * ring_stride;
   bool deferred = false;
   auto ensure_ring = [&] {
     if (nshift < 3) return;
-    const size_t one_field = r.data.bytes;
-    const bool have = mw.ring.size() == MS_DEFER - 1 && mw.ring[0].data.ptr && mw.ring[0].prec == P &&
-                      mw.ring[0].vh == vh && mw.ring[0].ls == ls;
-    if (!have) {
+    std::shared_ptr<DeviceBuffer> ring = L.ms_ring.lock();
+    if (!ring || ring->bytes < ring_bytes) {
       drop_graphs();
-      mw.ring.clear();
+      ring.reset();
+      mw.ring.reset();
       size_t free_b = 0, total_b = 0;
       CPSGPU_CUDA(cudaMemGetInfo(&free_b, &total_b));
-      if ((MS_DEFER - 1) * one_field > free_b / 4) return;
+      if (ring_bytes > free_b / 4) return;
       try {
-        mw.ring.resize(MS_DEFER - 1);
-        for (auto &f : mw.ring) f.create(P, vh, ls, 1);
+        ring = std::make_shared<DeviceBuffer>(ring_bytes);
       } catch (const Error &) {  // another allocation was first: no ring
         cudaGetLastError();
-        mw.ring.clear();
         return;
       }
+      L.ms_ring = ring;
+    }
+    if (mw.ring != ring) {
+      drop_graphs();
+      mw.ring = ring;
     }
     deferred = true;
   };
   const size_t per = (size_t)vh * ls;
   const size_t nvec = per * (P == PREC_DOUBLE ? 12 : 6);  // 16-byte elements of a field
-  auto slot_r = [&](int slot) { return slot == MS_DEFER - 1 ? r.view() : mw.ring[slot].view(); };
+  auto slot_r = [&](int slot) {
+    SpinorView v = r.view();
+    if (slot != MS_DEFER - 1) v.data = mw.ring->as<char>() + slot * ring_stride;
+    return v;
+  };
 
   // one iteration: M half (reduce <p,(A+m0)p>), M^dagger half with the
   // residual update, then the vector updates: of every shift (slot < 0), or
@@ -756,6 +765,10 @@ int minvcg(Dirac &D, double *const *psi_h, const double *chi_h, double chi_norm,
     t_ref = t_rec + std::chrono::duration_cast<clk::duration>(std::chrono::duration<double>(rec_ms * 1e-3));
   }
   const int iters = mh.k + 1;
+  if (mw.ring && mw.ring->bytes > ring_kept) {  // (the graph takes 3 ms to make, such a solve seconds)
+    drop_graphs();
+    mw.ring.reset();
+  }
 
   // FP64 view of solution k: the refined solution, else psi_k (converted
   // into tmp64 when it is FP32; used before the next call)

@@ -84,3 +84,35 @@ def test_larger_solves_on_the_lattice_between():
         busy.close()
         for a, b in zip(got, want):
             np.testing.assert_array_equal(a, b)
+
+
+def test_operators_of_one_lattice_share_the_ring():
+    """Operators of different Ls (the ring grows and moves), in turn, each call with the bits of its first; a second
+    operator takes no ring of its own, and the ring goes with the last of them."""
+    import torch
+
+    lat = Lattice((8, 8, 8, 16), (1, 1, 1, -1))
+    lat.import_gauge(gen_gauge((8, 8, 8, 16), seed=938))
+
+    def free():
+        return torch.cuda.mem_get_info()[0]
+
+    chis = {ls: gen_gaussian(24 * lat.vol // 2 * ls, seed=939 + ls) for ls in (8, 12, 4)}
+    ops = {ls: DiracOpDwf(lat, mass=0.1, ls=ls) for ls in chis}
+    first = {ls: _call(D, chis[ls], A.DOUBLE) for ls, D in ops.items()}
+    for ls in (4, 12, 8, 12, 4):
+        for a, b in zip(_call(ops[ls], chis[ls], A.DOUBLE), first[ls]):
+            np.testing.assert_array_equal(a, b)
+    for D in ops.values():
+        D.close()
+    ring = 7 * 192 * lat.vol // 2 * 12
+    start = free()
+    A1, B1 = DiracOpDwf(lat, mass=0.1, ls=12), DiracOpDwf(lat, mass=0.2, ls=12)
+    _call(A1, chis[12], A.DOUBLE)
+    one = start - free()
+    _call(B1, chis[12], A.DOUBLE)
+    two = start - free() - one
+    assert one - two > 0.9 * ring  # 66 MB
+    A1.close()
+    B1.close()
+    assert start - free() < 0.1 * ring
