@@ -48,9 +48,12 @@ dim3 hop_block(const TuneKey &k, bool mix) {
     // processes each: 16^3x32 Ls=16 FP32 498, 517 / 513, 525 us, FP16 437, 439
     // / 439, 441, FP64 901, 956 / 944, 939; 12x14x20x22 Ls=12 FP32 244, 242 /
     // 254, 248, FP16 213, 211 / 217, 215, FP64 427, 430 / 411, 411
-    if (k.ls % 4 == 0) return k.prec == PREC_DOUBLE ? dim3(32, 4) : dim3(64, 2);
-    // Ls = 6, 10, 14: an odd number of slices per parity, all of them
-    if (k.ls % 2 == 0 && k.ls <= 16) return dim3(32, k.ls / 2);
+    // Other even Ls, 64 x 2 / 32 x 2 (before) / 32 x Ls/2: 16^3x32 Ls=10 FP32 327 /
+    // 334 / 353, FP16 284 / 286 / 311, FP64 574 / 572 / 593, Ls=6 FP32 216 / 219 /
+    // 216, FP64 358 / 361 / 366; 16^4 Ls=14 FP32 252 / 257 / 266, FP16 224 / 227 /
+    // 237, FP64 407 / 403 / 440; 12^3x24 Ls=6 FP32 96 / 98 / 94
+    if (k.ls % 4 == 0 && k.prec == PREC_DOUBLE) return dim3(32, 4);
+    if (k.ls % 2 == 0) return dim3(64, 2);
   }
   int bs = (k.ls % 4 == 0) ? 4 : (k.ls % 2 == 0 ? 2 : 1);
   return dim3(32, bs);

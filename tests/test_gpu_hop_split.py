@@ -92,3 +92,20 @@ def test_batch_counts_all_its_sites(count):
         res.append([sol for _, sol, _ in items])
     assert all((a == b).all() for a, b in zip(*res)) == (count == 3)
     A.check(A.lib().cpsgpu_finalize())
+
+
+@pytest.mark.parametrize("prec", [A.DOUBLE, A.SINGLE, A.HALF])
+@pytest.mark.parametrize("ls", [2, 6, 10, 12, 14])
+def test_default_shape_of_larger_launches(ls, prec):
+    """above the rule's bound, with a partial last block of sites: the default shape's fields against one slice and 32
+    sites per block"""
+    L = {2: (10, 10, 10, 18), 6: (10, 6, 10, 14)}.get(ls, (10, 6, 6, 10))
+    u, lat, D = _op("dwf", L, ls)
+    x = gen_gaussian(D.f_size, seed=985)
+    default, dot = _fields(D, x, prec)
+    D.set_hop_shape(prec, 32, 1)
+    one, dot1 = _fields(D, x, prec)
+    for a, b in zip(default, one):
+        np.testing.assert_array_equal(a, b)
+    assert dot == pytest.approx(dot1, rel=1e-12)
+    A.check(A.lib().cpsgpu_finalize())
