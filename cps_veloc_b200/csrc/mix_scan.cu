@@ -137,10 +137,16 @@ __device__ __forceinline__ void unpack12(const Half12 &v, int lower, float2 (&f)
   for (int k = 0; k < 6; k++) f[k] = __half22float2(*reinterpret_cast<const __half2 *>(&w[k]));
 }
 
-// (the blocks per SM hold the registers where the loads in flight need them:
-// at Ls = 12 two blocks instead of three take 132 us instead of 109, 24^3x64)
+// blocks per SM that the registers have to allow: at Ls = 12 two instead of
+// three take 132 us instead of 109 (24^3x64), at 9 three instead of four 18.6
+// instead of 16.7 (16^3x32)
+template <int LS, bool BAND> constexpr int scan_half_blocks() {
+  if (BAND) return LS <= 8 ? 4 : LS <= 12 ? 3 : 2;
+  return LS <= 4 ? 6 : LS <= 6 ? 5 : LS <= 9 ? 4 : LS <= 12 ? 3 : 2;
+}
+
 template <int LS, bool BAND>
-__global__ void __launch_bounds__(SCAN_HALF_TPB, LS <= 8 ? 4 : LS <= 12 ? 3 : 2)
+__global__ void __launch_bounds__(SCAN_HALF_TPB, (scan_half_blocks<LS, BAND>()))
     scan_half_kernel(SpinorView in, SpinorView out, const ScanArg<float> arg, const SolverScalars *st, int gate, int rev) {
   if (gate == GATE_RUNNING && st[blockIdx.z].done) return;
   if (gate == GATE_RELIABLE && (st[blockIdx.z].done || !st[blockIdx.z].reliable)) return;
@@ -327,10 +333,12 @@ bool launch_mix_scan(const Dirac &D, int prec, const double *mix, const SpinorVi
   if (!m || in.ls != D.ls) return false;
   const cudaStream_t s = D.lat->stream;
   const int rev = D.lat->turn();
-  // the usual fifth extents in registers; others read the input twice (FP64,
-  // FP32), or take the dense kernels (FP16)
+  // up to Ls = 16 and the usual larger ones in registers (FP16 keeps LS / 2
+  // outputs too: up to 16 without spills); others read the input twice (FP64,
+  // FP32) or take the dense kernels (FP16).  M5^-1 on 16^3x32 in registers /
+  // otherwise, Ls = 5, 7, 11, 15: FP64 26 / 31, 33 / 43, 49 / 63, 64 / 87 us,
+  // FP32 14 / 14, 18 / 21, 25 / 30, 33 / 39, FP16 12 / 14, 14 / 21, 22 / 39, 33 / 62
   switch (D.ls) {
-  // (FP16 keeps LS / 2 outputs too: up to Ls = 16 without spills)
 #define CPSGPU_SCAN_LS(N)                                                                     \
   case N:                                                                                     \
     if (prec == PREC_DOUBLE) launch_full<PREC_DOUBLE, N>(*m, in, out, N, st, gate, s, rev);        \
@@ -338,13 +346,19 @@ bool launch_mix_scan(const Dirac &D, int prec, const double *mix, const SpinorVi
     else if constexpr (N <= 16) launch_half<N>(*m, in, out, st, gate, s, rev);                     \
     else return false;                                                                        \
     break;
+    CPSGPU_SCAN_LS(3)
     CPSGPU_SCAN_LS(4)
+    CPSGPU_SCAN_LS(5)
     CPSGPU_SCAN_LS(6)
+    CPSGPU_SCAN_LS(7)
     CPSGPU_SCAN_LS(8)
     CPSGPU_SCAN_LS(9)
     CPSGPU_SCAN_LS(10)
+    CPSGPU_SCAN_LS(11)
     CPSGPU_SCAN_LS(12)
+    CPSGPU_SCAN_LS(13)
     CPSGPU_SCAN_LS(14)
+    CPSGPU_SCAN_LS(15)
     CPSGPU_SCAN_LS(16)
     CPSGPU_SCAN_LS(20)
     CPSGPU_SCAN_LS(24)

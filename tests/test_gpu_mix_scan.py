@@ -38,7 +38,7 @@ def _check(D, ops, mass, prec, pieces=True):
 @pytest.mark.parametrize("L,ls", [((2, 2, 2, 2), 3), ((4, 2, 2, 2), 4), ((6, 2, 2, 2), 5), ((4, 4, 2, 2), 6),
                                   ((2, 2, 2, 6), 8), ((4, 6, 2, 2), 9), ((6, 6, 2, 2), 10), ((4, 4, 4, 4), 12),
                                   ((2, 6, 2, 6), 14), ((4, 2, 2, 10), 16), ((2, 2, 2, 4), 20), ((2, 2, 2, 2), 24),
-                                  ((2, 2, 2, 2), 32)])
+                                  ((2, 2, 2, 2), 32), ((4, 4, 2, 4), 7), ((2, 2, 6, 2), 11), ((4, 2, 2, 6), 13), ((2, 4, 2, 2), 15)])
 def test_recurrence(oracle, L, ls, prec):
     D, ops = _op(oracle, L, ls)
     _check(D, ops, 0.05, prec)
