@@ -112,9 +112,10 @@ struct Lattice {
   // first in turn, so that each starts on the part of its input that the one
   // before wrote last: with vectors of about the size of L2 (126 MB) that part
   // is still there.  No result depends on it (block partials are indexed by
-  // the sites).  Measured, forward only / in turn, CG us per iteration: Wilson
-  // 24^3x48 FP64 394.8 / 379.4, FP32 276 / 265, FP16 239.5 / 232.6; Mobius
-  // 16^3x32 Ls=12 FP32 463 / 453; DWF 24^3x64 and larger the same
+  // the sites).  Measured, forward only / in turn, CG us per iteration in FP64,
+  // FP32, FP16: Wilson 24^3x48 395 / 382, 271 / 260, 235 / 228; Mobius 16^3x32
+  // Ls=12 832 / 822, 453 / 444, 381 / 373; DWF 16^3x32 Ls=16 895 / 889, 494 / 487,
+  // 426 / 417
   int turn() const { return sweep.fetch_xor(1) & 1; }
   mutable std::atomic<int> sweep{0};
   GaugeView gauge(int prec) const;

@@ -145,9 +145,12 @@ __device__ __forceinline__ half_spinor<R> load_halo(const void *p, int face, lon
 // hop a basic block of its own, so the scheduler does not hoist the loads of
 // later directions until registers spill (FP64 hop: 176-352 B of spills in
 // one block, 32 B in four).  FP16 storage keeps one block: its loads are few
-// and the hoisting pays there.  Measured, MatPcDagMatPc on DWF 16^3x32 Ls=16:
-// FP64 692 -> 665 us, FP32 362 -> 350 us (FP16 332 -> 344: not used); Wilson
-// 24^3x48 FP32 200 -> 189 us.
+// and the hoisting pays there (332 -> 344 us with four: not used).  Measured,
+// one block / four, MatPcDagMatPc and CG iteration in us: FP64 DWF 16^3x32 Ls=16
+// 689 / 664 and 944 / 889, Wilson 24^3x48 320 / 306 and 399 / 382, Mobius
+// 16^3x32 Ls=12 696 / 675 and 852 / 822; FP32 Mobius 364 / 355 and 453 / 444,
+// Wilson 182 / 181 and 262 / 260, and DWF 353 / 360 and 482 / 487, where it
+// costs a little (Wilson and DWF are one instantiation).
 template <int P> __device__ __forceinline__ bool own_block(const HopParams &hp, int mu) {
   return P == PREC_HALF || hp.ls > -mu;
 }

@@ -29,10 +29,10 @@
 // sites, a thread holding the 12 stored values of every slice of its site
 // and the site's norms; the new norm is the larger of the two chiralities'
 // maxima (shuffles).  Measured (M5^-1, 24^3x64, Ls = 12, dense
-// kernel before / this): FP64 467 / 327 us (6.2 TB/s), FP32 191 / 160 us
-// (6.4 TB/s), FP16 174 / 111 us (5.0 TB/s); MatPcDagMatPc, with the hop's
-// mixing epilogue in the same form: FP64 5.89 / 5.42 ms, FP32 2.56 / 2.35 ms,
-// FP16 2.11 / 1.83 ms
+// kernel / this): FP64 467 / 330 us (6.2 TB/s), FP32 193 / 160 us
+// (6.4 TB/s), FP16 174 / 110 us (5.0 TB/s); MatPcDagMatPc, with the hop's
+// mixing epilogue in the same form: FP64 5.80 / 5.43 ms, FP32 2.53 / 2.26 ms,
+// FP16 2.11 / 1.81 ms
 #include <cmath>
 
 #include "cpsgpu_impl.h"

@@ -81,10 +81,11 @@ def test_several_right_hand_sides():
             assert r.status == A.CONVERGED and r.true_res <= 1e-10
 
 
-@pytest.mark.parametrize("b,c,ls", [(1.45, 0.45, 12), (1.0, 0.4545, 8), (1.5, 0.5, 10), (2.5, 1.5, 16), (4.0, 3.0, 6)])
+@pytest.mark.parametrize("b,c,ls", [(1.45, 0.45, 12), (1.0, 0.4545, 8), (1.5, 0.5, 10), (2.5, 1.5, 16), (4.0, 3.0, 6),
+                                    (4.5, 3.5, 10)])
 def test_precision_of_the_form(oracle, b, c, ls):
-    """K from -2e-5 over 0.02 to 0.57: no term of the recurrence may be larger than the matrix (c / |K| is up to 2e4
-    here).  MatPcDagMatPc is four mixings and four hops; a mixing's error is below 7e-8 in FP32 and 2e-16 in FP64 (the
+    """K from -2e-5 over 0.02 to 0.57 and, dense, 0.62: no term of the recurrence may be larger than the matrix (c / |K|
+    is up to 2e4 here).  MatPcDagMatPc is four mixings and four hops; a mixing's error is below 7e-8 in FP32 and 2e-16 in FP64 (the
     roundings of its coefficients and three operations), a hop's below 1.2e-7 and 2.5e-16 (the 2-norm of 8 sums of
     products of unit roundoff 6e-8 and 1.1e-16), and the oracle's as FP64's: 8e-7 and 4e-15 in all."""
     D, ops = _op(oracle, (4, 4, 4, 4), ls, b, c)
