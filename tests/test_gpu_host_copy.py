@@ -36,8 +36,8 @@ def test_a_lattice_per_configuration():
     other = Lattice(L)
     beside = make()
     other.close()
-    # 18 and 2.7 ms where each lattice pins and frees its buffers
-    assert alone < 2.5 * beside + 2e-3
+    # 6.7 and 2.8 ms; 18-22 and 2.8 where each lattice pins and frees its buffers
+    assert alone < 3 * beside + 4e-3
 
 
 @pytest.mark.parametrize("sizes", [((4, 4, 4, 4), 1), ((4, 4, 8, 8), 3), ((8, 8, 8, 8), 8)])
